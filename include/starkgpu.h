@@ -651,7 +651,7 @@ SG_API int sg_rv64_memory_table(sg_ctx* ctx, void* stream, const uint64_t* cells
  *      its device time), oldest first, then clears the log. ---- */
 typedef struct {
     uint32_t log_len;  /* points per tile, log2 */
-    uint32_t cols;     /* tile width (columns per tile) */
+    uint32_t cols;     /* tile width (columns per tile); 0: the pass ran on the tensor cores */
     uint32_t inverse;  /* 1: inverse transform */
     uint32_t reps;     /* coset repetitions per tile (blowup for the LDE's first forward pass) */
     uint32_t pre;      /* 1: per-point coset-shift factors before the transform */

@@ -199,6 +199,21 @@ int sg_ctx_create(int device, uint64_t budget, sg_ctx** out) {
         uint64_t thr = ctx->budget;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
+    void* word = nullptr;
+    void* dev_word = nullptr;
+    cudaError_t e = cudaHostAlloc(&word, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable);
+    if (e == cudaSuccess) {
+        *(unsigned*)word = 0;
+        ctx->fault_host = (volatile unsigned*)word;
+        e = cudaHostGetDevicePointer(&dev_word, word, 0);
+        ctx->fault_dev = (unsigned*)dev_word;
+    }
+    if (e != cudaSuccess) {
+        if (word) cudaFreeHost(word);
+        delete ctx;
+        set_error(std::string("context error word: ") + cudaGetErrorString(e));
+        return e == cudaErrorMemoryAllocation ? SG_ERR_OOM : SG_ERR_CUDA;
+    }
     *out = reinterpret_cast<sg_ctx*>(ctx);
     return SG_OK;
 }
@@ -215,6 +230,7 @@ void sg_ctx_destroy(sg_ctx* c) {
     for (auto e : ctx->stage_free)
         if (e) cudaEventDestroy(e);
     if (ctx->stage) cudaFreeHost(ctx->stage);
+    if (ctx->fault_host) cudaFreeHost((void*)ctx->fault_host);
     delete ctx;
 }
 
@@ -269,7 +285,7 @@ int sg_stream_sync(sg_ctx* c, void* stream) {
     SG_CHECK_ARG(c, "null context");
     SG_ENTER(ctx_of(c));
     SG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    return SG_OK;
+    return check_fault(C(c));
 }
 
 int sg_stream_create(sg_ctx* c, void** out) {

@@ -114,6 +114,11 @@ struct Ctx {
     std::vector<PassLog> passlog;
     // Learned pass-cost model (mlp.cu): when set, DFT tile widths are its choice.
     std::vector<float> pass_model;
+    // One page-locked word that a kernel sets when a bounded wait of its ran
+    // out (ntt_tc.cu); null in contexts that do not allocate. The launch check
+    // and sg_stream_sync report it.
+    volatile unsigned* fault_host = nullptr;
+    unsigned* fault_dev = nullptr;
 };
 
 // Host-side prediction of the pass-cost model (mlp.cu): log(ms) for features x.
@@ -189,6 +194,15 @@ struct KernelInfo {
 };
 int kernel_info(const void* fn, size_t smem, int threads, KernelInfo* out);
 
+// An earlier kernel of the context gave up a bounded wait: its output is not valid.
+inline int check_fault(Ctx* ctx) {
+    if (ctx->fault_host && *ctx->fault_host) {
+        set_error("a kernel of this context gave up waiting for its tensor-core products");
+        return SG_ERR_CUDA;
+    }
+    return SG_OK;
+}
+
 inline int check_launch(Ctx* ctx, const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -196,7 +210,7 @@ inline int check_launch(Ctx* ctx, const char* what) {
         return SG_ERR_CUDA;
     }
     ctx->launches.fetch_add(1, std::memory_order_relaxed);
-    return SG_OK;
+    return check_fault(ctx);
 }
 
 // ---- internal kernel drivers (ntt.cu, merkle.cu) ----

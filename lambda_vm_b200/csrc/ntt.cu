@@ -32,6 +32,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "dft.cuh"
 #include "gl.cuh"
 
 namespace sg {
@@ -89,47 +90,6 @@ __device__ __forceinline__ uint32_t brev_q(uint32_t r) {
     else
         return __brev(r) >> (32 - Q);
 }
-
-// omega_N^e = lo[e & (2^h - 1)] * hi[e >> h], N = 2^logN.
-struct Tw {
-    const uint64_t* lo;
-    const uint64_t* hi;
-    uint32_t h;
-    uint32_t logN;
-};
-
-__device__ __forceinline__ uint64_t tw_pow(const Tw& t, uint64_t e) {
-    return gl::mul(__ldg(t.lo + (e & ((1ULL << t.h) - 1))), __ldg(t.hi + (e >> t.h)));
-}
-
-// omega_{2^logM}^{+-x}
-__device__ __forceinline__ uint64_t tw_root(const Tw& t, uint32_t logM, uint64_t x, bool inv) {
-    const uint64_t mask = (1ULL << t.logN) - 1;
-    uint64_t e = (x << (t.logN - logM)) & mask;
-    if (inv) e = (mask + 1 - e) & mask;
-    return tw_pow(t, e);
-}
-
-struct PassArgs {
-    const uint64_t* in;
-    uint64_t* out;
-    uint64_t m;               // columns transformed
-    uint64_t in_ld, out_ld;   // row strides of in / out in u64 (>= m)
-    uint32_t logL;
-    uint32_t inverse;
-    // row(tile, point, rep) = tile*ts + point*ps + rep*rs
-    uint64_t in_ts, in_ps;
-    uint64_t out_ts, out_ps, out_rs;
-    uint32_t reps;
-    Tw tw;
-    uint32_t pre_kind;   // 0: none, 1: omega_{2^pre_log}^{in_row * rep}
-    uint32_t pre_log;
-    uint32_t post_kind;  // 0: none, 1: omega_{2^post_log}^{+-(tile*k)}, 2: weights[out_row], 3: scalar
-    uint32_t post_log;
-    const uint64_t* weights;
-    uint64_t scalar;
-    uint32_t canon_out;
-};
 
 // Compile-time stage plan per tile: 2^LOGL points x CC columns. A tile runs
 // NST register stages of at most 2^QM points each (larger radices first):
@@ -591,13 +551,16 @@ static int tune_tiles(Ctx* ctx, cudaStream_t st, uint32_t logL) {
     return rc != SG_OK ? rc : rf;
 }
 
+// The columns of a pass's tiles, or 0 when the pass runs on the tensor cores:
+// every pass dft_tc_takes, unless the context pins this length's width or may
+// not allocate (it then has no error word for the kernel's bounded waits).
 static int pick_cols(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntiles, int* cols) {
     const uint32_t logL = a.logL;
     const uint64_t m = a.m;
     int vs[4];
     const int nv = tile_variants(logL, vs);
     *cols = default_cols((int)logL);
-    if (nv == 1 || !ctx->autotune) return SG_OK;
+    if (!ctx->autotune) return SG_OK;
     {
         std::lock_guard<std::mutex> g(ctx->tune_mu);
         const int forced = ctx->tiles[logL].forced;
@@ -605,6 +568,11 @@ static int pick_cols(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntil
             *cols = forced;
             return SG_OK;
         }
+        if (ctx->fault_dev && dft_tc_takes(a, ntiles)) {
+            *cols = 0;
+            return SG_OK;
+        }
+        if (nv == 1) return SG_OK;
         // With a learned pass-cost model installed, each compiled width's pass
         // time is predicted from the pass's shape and the fastest is taken; no
         // timing probe runs.
@@ -639,10 +607,14 @@ static int pick_cols(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntil
     return SG_OK;
 }
 
+static int launch_pass(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntiles, int cols) {
+    return cols ? launch_cols(ctx, st, a, ntiles, cols) : launch_dft_tc(ctx, st, a, ntiles);
+}
+
 static int run_pass(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntiles) {
     int cols = 0;
     SG_TRY(pick_cols(ctx, st, a, ntiles, &cols));
-    if (!ctx->passlog_on.load(std::memory_order_relaxed)) return launch_cols(ctx, st, a, ntiles, cols);
+    if (!ctx->passlog_on.load(std::memory_order_relaxed)) return launch_pass(ctx, st, a, ntiles, cols);
     // pass log: the launch between two events, read back by sg_ctx_pass_log_read
     Ctx::PassLog r{};
     r.rec.log_len = a.logL, r.rec.cols = (uint32_t)cols, r.rec.inverse = a.inverse, r.rec.reps = a.reps;
@@ -651,7 +623,7 @@ static int run_pass(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntile
     SG_CUDA(cudaEventCreate(&r.e0));
     cudaError_t e = cudaEventCreate(&r.e1);
     if (e == cudaSuccess) e = cudaEventRecord(r.e0, st);
-    int rc = e == cudaSuccess ? launch_cols(ctx, st, a, ntiles, cols) : SG_ERR_CUDA;
+    int rc = e == cudaSuccess ? launch_pass(ctx, st, a, ntiles, cols) : SG_ERR_CUDA;
     if (rc == SG_OK) e = cudaEventRecord(r.e1, st);
     if (e != cudaSuccess || rc != SG_OK) {
         if (e != cudaSuccess) set_error(std::string("pass log: ") + cudaGetErrorString(e));
@@ -954,6 +926,11 @@ int lde_multi(Ctx* ctx, cudaStream_t st, const LdeJob* jobs, uint32_t count) {
     std::vector<Group> groups;
     for (size_t i = 0; i < plan.size(); ++i) {
         const Planned& p = plan[i];
+        if (p.cols == 0) {  // a tensor-core pass is a launch of its own
+            groups.push_back({i, i + 1, 0});
+            descs[i] = PassDesc{};
+            continue;
+        }
         if (groups.empty() || p.step != plan[groups.back().begin].step || p.a.logL != plan[groups.back().begin].a.logL ||
             p.cols != plan[groups.back().begin].cols || p.a.inverse != plan[groups.back().begin].a.inverse)
             groups.push_back({i, i, 0});
@@ -975,6 +952,10 @@ int lde_multi(Ctx* ctx, cudaStream_t st, const LdeJob* jobs, uint32_t count) {
     for (const Group& g : groups) {
         if (rc != SG_OK) break;
         const Planned& p = plan[g.begin];
+        if (p.cols == 0) {
+            rc = launch_dft_tc(ctx, st, p.a, p.ntiles);
+            continue;
+        }
         rc = launch_multi_cols(ctx, st, p.a.logL, p.cols, p.a.inverse != 0, d_descs + g.begin,
                                (uint32_t)(g.end - g.begin), g.total);
     }
