@@ -54,55 +54,23 @@ __device__ __forceinline__ bool is_zero3(fe3 v) {
 // inversion is a serial chain the other lanes wait on, so a warp covers
 // 32 * BI_CH elements to spread it (and the scans) thin; the unwind reloads
 // the inputs instead of holding them in registers, each before its own
-// output is stored (the inversion may run in place). 2^22 x 3 DEEP
-// denominators: 4 elements a thread 1.24 ms, 8: 0.82, 12: 0.72, 16: 1.24
-// (153 registers, one block per SM); one inversion per block instead of per
-// warp: 0.79 (the block waits on one thread's chain).
+// output is stored (the inversion may run in place). 2^22 x 3 elements: 4 a
+// thread 1.24 ms, 8: 0.82, 12: 0.72, 16: 1.24 (153 registers, one block per
+// SM); one inversion per block instead of per warp: 0.79 (the block waits on
+// one thread's chain).
 #define BI_CH 12
 
-struct LoadPlain {
-    const uint64_t* in;
-    struct Cur {
-        uint64_t base;
-    };
-    __device__ __forceinline__ Cur start(uint64_t base) const { return Cur{base}; }
-    __device__ __forceinline__ fe3 at(const Cur& c, int j) const { return ld3(in + 3 * (c.base + j)); }
-};
-// Denominators z_k - x_i (sign 0) or x_i - z_k (sign 1), element idx = k*n + i.
-// A thread's cursor divides once; its later elements step (k, i) forward.
-struct LoadDenom {
-    const uint64_t* x;
-    const uint64_t* z;
-    uint64_t n;
-    int x_minus_z;
-    struct Cur {
-        uint64_t k, i;
-    };
-    __device__ __forceinline__ Cur start(uint64_t base) const {
-        const uint64_t k = base / n;
-        return Cur{k, base - k * n};
-    }
-    __device__ __forceinline__ fe3 at(const Cur& c, int j) const {
-        uint64_t k = c.k, i = c.i + (uint64_t)j;
-        while (i >= n) i -= n, ++k;
-        const fe3 zk = ld3(z + 3 * k);
-        const uint64_t xi = x[i];
-        return x_minus_z ? fe3{gl::sub(xi, zk.c0), gl::neg(zk.c1), gl::neg(zk.c2)}
-                         : fe3{gl::sub(zk.c0, xi), zk.c1, zk.c2};
-    }
-};
-
-template <class Load>
-__global__ void __launch_bounds__(256) k_batch_inv(Load load, uint64_t total, uint64_t* out, unsigned* zero_flag) {
+__global__ void __launch_bounds__(256) k_batch_inv(const uint64_t* in, uint64_t total, uint64_t* out,
+                                                   unsigned* zero_flag) {
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t base = tid * BI_CH;
     const int lane = threadIdx.x & 31;
-    const typename Load::Cur cur = load.start(base < total ? base : 0);
+    auto at = [&](int j) { return ld3(in + 3 * (base + j)); };
     // prefix products of the chunk; elements past the end count as 1
     fe3 p[BI_CH];
-    p[0] = base < total ? load.at(cur, 0) : one3();
+    p[0] = base < total ? at(0) : one3();
 #pragma unroll
-    for (int i = 1; i < BI_CH; ++i) p[i] = base + i < total ? gl::mul3(p[i - 1], load.at(cur, i)) : p[i - 1];
+    for (int i = 1; i < BI_CH; ++i) p[i] = base + i < total ? gl::mul3(p[i - 1], at(i)) : p[i - 1];
     const fe3 tot = p[BI_CH - 1];
     fe3 incl = tot, sinc = tot;
 #pragma unroll
@@ -128,7 +96,7 @@ __global__ void __launch_bounds__(256) k_batch_inv(Load load, uint64_t total, ui
 #pragma unroll
     for (int i = BI_CH - 1; i >= 1; --i) {
         if (base + i < total) {
-            const fe3 a = load.at(cur, i);  // before the store: out may alias the input
+            const fe3 a = at(i);  // before the store: out may alias the input
             st3(out + 3 * (base + i), gl::canon3(gl::mul3(inv, p[i - 1])));
             inv = gl::mul3(inv, a);
         }
@@ -136,9 +104,10 @@ __global__ void __launch_bounds__(256) k_batch_inv(Load load, uint64_t total, ui
     if (base < total) st3(out + 3 * base, gl::canon3(inv));
 }
 
-template <class Load>
-static int batch_inv_launch(Ctx* ctx, cudaStream_t st, Load load, uint64_t total, uint64_t* out, int* zero_out) {
-    if (total == 0) return SG_OK;
+// Run `launch(flag)` with a zeroed device flag word; the flag it leaves goes to
+// *zero_out when that is wanted (the call then waits for it).
+template <class F>
+static int with_zero_flag(Ctx* ctx, cudaStream_t st, int* zero_out, F&& launch) {
     unsigned* d_flag = nullptr;
     SG_TRY(dev_alloc(ctx, st, sizeof(unsigned), (void**)&d_flag));
     int rc = SG_OK;
@@ -146,11 +115,7 @@ static int batch_inv_launch(Ctx* ctx, cudaStream_t st, Load load, uint64_t total
         set_error("batch inverse: flag reset failed");
         rc = SG_ERR_CUDA;
     }
-    if (rc == SG_OK) {
-        const uint64_t threads = (total + BI_CH - 1) / BI_CH;
-        k_batch_inv<Load><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(load, total, out, d_flag);
-        rc = check_launch(ctx, "k_batch_inv");
-    }
+    if (rc == SG_OK) rc = launch(d_flag);
     if (rc == SG_OK && zero_out) {
         unsigned h = 0;
         if (cudaMemcpyAsync(&h, d_flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -165,6 +130,100 @@ static int batch_inv_launch(Ctx* ctx, cudaStream_t st, Load load, uint64_t total
 }
 
 // ---------------------------------------------------------------- barycentric sums
+static int batch_inv_launch(Ctx* ctx, cudaStream_t st, const uint64_t* in, uint64_t total, uint64_t* out,
+                            int* zero_out) {
+    if (total == 0) return SG_OK;
+    return with_zero_flag(ctx, st, zero_out, [&](unsigned* d_flag) {
+        const uint64_t threads = (total + BI_CH - 1) / BI_CH;
+        k_batch_inv<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(in, total, out, d_flag);
+        return check_launch(ctx, "k_batch_inv");
+    });
+}
+
+// Inverses of the denominators z_k - x_i (x_minus_z 0) or x_i - z_k (1) with
+// base-field points x: an element is (u, a1, a2) with u = +-(x_i - z_k0) and
+// a1, a2 constant in i, so with the norm's coefficients folded once per k,
+//   N(u) = u (u^2 - 6 a1 a2) + 2 a1^3 + 4 a2^3,
+//   inverse = (u^2 - 2 a1 a2, 2 a2^2 - a1 u, a1^2 - a2 u) / N,
+// and Montgomery's trick runs on the base-field norms: 11 base products an
+// element where inverting ext3 elements took three ext3 products (27).
+// Bound by integer issue. A warp takes 32 CH consecutive points of one k,
+// thread `lane` the points lane, lane + 32, ...: points are read and results
+// written (through shared memory) in whole segments; a warp prefix and suffix
+// scan of the threads' products leaves one base-field inversion a warp.
+// CH: 16 where that fills the schedulers, 4 below (a thread's chain is the
+// latency there).
+template <int CH>
+__global__ void __launch_bounds__(256) k_inv_denoms(const uint64_t* __restrict__ x, const uint64_t* __restrict__ z,
+                                                    uint64_t n, int x_minus_z, uint64_t* __restrict__ out,
+                                                    unsigned* zero_flag) {
+    __shared__ uint64_t cst[8], stage[8][96];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t* zk = z + 3 * (uint64_t)blockIdx.y;
+    if (threadIdx.x == 0) {
+        const uint64_t a1 = x_minus_z ? gl::neg(zk[1]) : zk[1], a2 = x_minus_z ? gl::neg(zk[2]) : zk[2];
+        const uint64_t a11 = gl::sqr(a1), a22 = gl::sqr(a2), p = gl::mul(a1, a2), c = gl::add(p, p);
+        const uint64_t t = gl::add(gl::mul(a11, a1), gl::mul(gl::add(a22, a22), a2));
+        cst[0] = zk[0], cst[1] = a1, cst[2] = a2, cst[3] = c;
+        cst[4] = gl::add(a22, a22), cst[5] = a11, cst[6] = gl::add(gl::add(c, c), c), cst[7] = gl::add(t, t);
+    }
+    __syncthreads();
+    const uint64_t z0 = cst[0], a1 = cst[1], a2 = cst[2];
+    const uint64_t base = ((uint64_t)blockIdx.x * 8 + warp) * (32 * CH);
+    if (base >= n) return;  // warp-uniform
+    auto u_of = [&](int j) {
+        const uint64_t xi = __ldg(x + base + 32 * j + lane);
+        return x_minus_z ? gl::sub(xi, z0) : gl::sub(z0, xi);
+    };
+    // norms, and the prefix products of the thread's; points past the end count as 1
+    uint64_t N[CH], p[CH];
+#pragma unroll
+    for (int j = 0; j < CH; ++j) {
+        N[j] = 1;
+        if (base + 32 * j + lane < n) {
+            const uint64_t u = u_of(j);
+            N[j] = gl::add(gl::mul(u, gl::sub(gl::sqr(u), cst[6])), cst[7]);
+        }
+        p[j] = j ? gl::mul(p[j - 1], N[j]) : N[j];
+    }
+    uint64_t incl = p[CH - 1], sinc = p[CH - 1];
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint64_t v = __shfl_up_sync(0xffffffffu, incl, off), w = __shfl_down_sync(0xffffffffu, sinc, off);
+        if ((int)lane >= off) incl = gl::mul(v, incl);
+        if ((int)lane + off < 32) sinc = gl::mul(sinc, w);
+    }
+    uint64_t excl = __shfl_up_sync(0xffffffffu, incl, 1), sexcl = __shfl_down_sync(0xffffffffu, sinc, 1);
+    if (lane == 0) excl = 1;
+    if (lane == 31) sexcl = 1;
+    uint64_t tinv = 0;
+    if (lane == 31) {  // the warp's product
+        if (gl::canon(incl) == 0) atomicOr(zero_flag, 1u);
+        tinv = gl::inv(gl::canon(incl));
+    }
+    tinv = __shfl_sync(0xffffffffu, tinv, 31);
+    uint64_t inv = gl::mul(gl::mul(tinv, sexcl), excl);  // of the thread's product
+    uint64_t* o = out + 3 * ((uint64_t)blockIdx.y * n + base);
+#pragma unroll
+    for (int j = CH - 1; j >= 0; --j) {
+        const uint64_t ninv = j ? gl::mul(inv, p[j - 1]) : inv;
+        if (j) inv = gl::mul(inv, N[j]);
+        const uint64_t left = n - base > 32ull * j ? n - base - 32ull * j : 0;  // points from this row on
+        if (lane < left) {
+            const uint64_t u = u_of(j);
+            uint64_t* q = stage[warp] + 3 * lane;
+            q[0] = gl::canon(gl::mul(gl::sub(gl::sqr(u), cst[3]), ninv));
+            q[1] = gl::canon(gl::mul(gl::sub(cst[4], gl::mul(a1, u)), ninv));
+            q[2] = gl::canon(gl::mul(gl::sub(cst[5], gl::mul(a2, u)), ninv));
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t w = lane; w < 96; w += 32)
+            if (w < 3 * left) o[96ull * j + w] = stage[warp][w];
+        __syncwarp();
+    }
+}
+
 // out_partial[(chunk * K + k) * cols + c] = sum over the chunk's rows i of
 //   points[i] * col_c(row i*stride) * inv_denoms[k][i]
 #define BARY_MAX_K 8
@@ -592,7 +651,7 @@ int sg_batch_inverse_ext3(sg_ctx* c, void* stream, const uint64_t* d_in, uint64_
                           int* zero_found) {
     SG_CHECK_ARG(c && (n == 0 || (d_in && d_out)), "null argument");
     SG_ENTER(ctx_of(c));
-    return batch_inv_launch(CX(c), (cudaStream_t)stream, LoadPlain{d_in}, n, d_out, zero_found);
+    return batch_inv_launch(CX(c), (cudaStream_t)stream, d_in, n, d_out, zero_found);
 }
 
 int sg_inv_denoms_ext3(sg_ctx* c, void* stream, const uint64_t* d_x, uint64_t n, const uint64_t* z_host, uint32_t k,
@@ -609,7 +668,23 @@ int sg_inv_denoms_ext3(sg_ctx* c, void* stream, const uint64_t* d_x, uint64_t n,
         set_error("inv_denoms: z upload failed");
         rc = SG_ERR_CUDA;
     }
-    if (rc == SG_OK) rc = batch_inv_launch(ctx, st, LoadDenom{d_x, d_z, n, x_minus_z}, n * k, d_out, zero_found);
+    if (rc == SG_OK)
+        rc = with_zero_flag(ctx, st, zero_found, [&](unsigned* d_flag) {
+            // 16 points a thread once that gives every scheduler a few warps
+            const bool wide = n * k >= (1ULL << 20);
+            const uint64_t per = 256ull * (wide ? 16 : 4);
+            for (uint32_t k0 = 0; k0 < k; k0 += 65535) {  // grid.y limit
+                const dim3 grid((unsigned)((n + per - 1) / per), k - k0 < 65535 ? k - k0 : 65535);
+                const uint64_t* zp = d_z + 3ull * k0;
+                uint64_t* o = d_out + 3ull * k0 * n;
+                if (wide)
+                    k_inv_denoms<16><<<grid, 256, 0, st>>>(d_x, zp, n, x_minus_z, o, d_flag);
+                else
+                    k_inv_denoms<4><<<grid, 256, 0, st>>>(d_x, zp, n, x_minus_z, o, d_flag);
+                SG_TRY(check_launch(ctx, "k_inv_denoms"));
+            }
+            return SG_OK;
+        });
     int rf = dev_free(ctx, st, d_z, 24ull * k);
     return rc != SG_OK ? rc : rf;
 }
@@ -845,7 +920,7 @@ int sg_logup_aux(sg_ctx* c, void* stream, const uint64_t* d_main, uint64_t n, ui
             k_logup_fp<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(d_main, n, m, d, z[0], z[1], z[2], d_fp);
             rc = check_launch(ctx, "k_logup_fp");
             int zf = 0;
-            if (rc == SG_OK) rc = batch_inv_launch(ctx, st, LoadPlain{d_fp}, tot, d_fp, &zf);
+            if (rc == SG_OK) rc = batch_inv_launch(ctx, st, d_fp, tot, d_fp, &zf);
             if (rc == SG_OK && zf) {
                 set_error("logup: a fingerprint is zero (challenge collides with a row value)");
                 rc = SG_ERR_INVALID;

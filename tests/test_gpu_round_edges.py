@@ -1,0 +1,34 @@
+"""Sizes at which the round kernels change form, against the CPU oracle: runs
+of 16 or 4 denominators a thread, more LogUp segments than scanning threads,
+two lanes or one thread a sponge (FRI layers, leaves, tree levels)."""
+import numpy as np
+import pytest
+
+import oracle as O
+from lambda_vm_b200 import math_cuda as mc
+from lambda_vm_b200.air import SynthTableAir
+
+pytestmark = pytest.mark.gpu
+P = O.P
+
+
+def rf(rng, shape):
+    x = rng.integers(0, 2**64, size=shape, dtype=np.uint64)
+    return np.where(x >= np.uint64(P), x - np.uint64(P), x)
+
+
+# 2^20 denominators and more run 16 a thread (512 a warp), fewer 4 (128 a warp)
+@pytest.mark.parametrize("n,k,sign", [(127, 2, 0), (129, 3, 1), (1024, 1, 0), (1 << 20, 1, 1), ((1 << 19) + 1, 2, 0),
+                                      ((1 << 20) - 511, 2, 1), (300007, 5, 0)])
+def test_denominators(be, n, k, sign):
+    rng = np.random.default_rng(n + k)
+    x, z = rf(rng, (n,)), rf(rng, (k, 3))
+    z[0, 1:] = 0  # a base-field point: the norm's constants vanish
+    got = mc.compute_and_invert_denoms_ext3(x, z, sign, be)
+    assert (got == O.canon_array(O.inv_denoms(x, z, sign))).all()
+
+
+def test_zero_denominator_is_reported(be):
+    x = np.arange(1, 5001, dtype=np.uint64)
+    with pytest.raises(ZeroDivisionError):
+        mc.compute_and_invert_denoms_ext3(x, np.array([[7, 1, 2], [4321, 0, 0]], np.uint64), 1, be)
