@@ -129,7 +129,6 @@ static int with_zero_flag(Ctx* ctx, cudaStream_t st, int* zero_out, F&& launch) 
     return rc != SG_OK ? rc : rf;
 }
 
-// ---------------------------------------------------------------- barycentric sums
 static int batch_inv_launch(Ctx* ctx, cudaStream_t st, const uint64_t* in, uint64_t total, uint64_t* out,
                             int* zero_out) {
     if (total == 0) return SG_OK;
@@ -225,6 +224,7 @@ __global__ void __launch_bounds__(256) k_inv_denoms(const uint64_t* __restrict__
 }
 
 // out_partial[(chunk * K + k) * cols + c] = sum over the chunk's rows i of
+// ---------------------------------------------------------------- barycentric sums
 //   points[i] * col_c(row i*stride) * inv_denoms[k][i]
 #define BARY_MAX_K 8
 #define BARY_PF 4  // rows in flight per thread: 4, 8, 16 measured 1.60, 1.79, 1.78 ms (2^20 x 256, K = 2)
@@ -595,18 +595,43 @@ __global__ void __launch_bounds__(256) k_seg_sum(const uint64_t* rsum, uint64_t 
     }
 }
 
-// Exclusive prefix of the segment sums, total L and offset L/n (one thread:
-// at most n/1024 segments).
-__global__ void k_seg_scan(uint64_t* seg, uint64_t nseg, uint64_t ninv, uint64_t* L_off) {
-    if (threadIdx.x || blockIdx.x) return;
-    fe3 run = zero3();
-    for (uint64_t s = 0; s < nseg; ++s) {
+// Exclusive prefix of the segment sums, total L and offset L/n. One CTA, each
+// thread a run of consecutive segments (one thread's chain of loads and
+// additions over all of them took 145 us at 1024 segments).
+__global__ void __launch_bounds__(1024) k_seg_scan(uint64_t* seg, uint64_t nseg, uint64_t ninv, uint64_t* L_off) {
+    __shared__ uint64_t wsum[3 * 32];
+    const uint64_t per = (nseg + blockDim.x - 1) / blockDim.x;
+    const uint64_t s0 = min(nseg, threadIdx.x * per), s1 = min(nseg, s0 + per);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    fe3 own = zero3();
+    for (uint64_t s = s0; s < s1; ++s) own = gl::add3(own, ld3(seg + 3 * s));
+    fe3 incl = own;
+    for (int off = 1; off < 32; off <<= 1) {
+        const fe3 u = shfl_up3(incl, off);
+        if (lane >= off) incl = gl::add3(incl, u);
+    }
+    if (lane == 31) st3(wsum + 3 * w, incl);
+    __syncthreads();
+    if (w == 0) {
+        const fe3 x = ld3(wsum + 3 * lane);
+        fe3 xi = x;
+        for (int off = 1; off < 32; off <<= 1) {
+            const fe3 u = shfl_up3(xi, off);
+            if (lane >= off) xi = gl::add3(xi, u);
+        }
+        if (lane == 31) {
+            st3(L_off, gl::canon3(xi));
+            st3(L_off + 3, gl::mulb3(xi, ninv));
+        }
+        st3(wsum + 3 * lane, gl::sub3(xi, x));  // exclusive warp prefix
+    }
+    __syncthreads();
+    fe3 run = gl::add3(ld3(wsum + 3 * w), gl::sub3(incl, own));
+    for (uint64_t s = s0; s < s1; ++s) {
         const fe3 v = ld3(seg + 3 * s);
         st3(seg + 3 * s, run);
         run = gl::add3(run, v);
     }
-    st3(L_off, gl::canon3(run));
-    st3(L_off + 3, gl::mulb3(run, ninv));
 }
 
 // acc[r] = (sum_{r' < r} rsum[r']) - r * (L / n), written to aux column W-1.
@@ -936,7 +961,7 @@ int sg_logup_aux(sg_ctx* c, void* stream, const uint64_t* d_main, uint64_t n, ui
         }
         if (rc == SG_OK) {
             const uint64_t ninv = sg_host_gl_inv(n % GL_P);
-            k_seg_scan<<<1, 32, 0, st>>>(d_seg + 6, nseg, ninv, d_seg);
+            k_seg_scan<<<1, 1024, 0, st>>>(d_seg + 6, nseg, ninv, d_seg);
             rc = check_launch(ctx, "k_seg_scan");
         }
         if (rc == SG_OK) {

@@ -32,3 +32,17 @@ def test_zero_denominator_is_reported(be):
     x = np.arange(1, 5001, dtype=np.uint64)
     with pytest.raises(ZeroDivisionError):
         mc.compute_and_invert_denoms_ext3(x, np.array([[7, 1, 2], [4321, 0, 0]], np.uint64), 1, be)
+
+
+# 1024-row segments: one a scanning thread up to 2^20 rows, two and three above
+@pytest.mark.parametrize("n", [1, 1024, 1025, 1 << 20, (1 << 20) + 5, (1 << 21) + 1024])
+def test_logup_segments(be, n):
+    rng = np.random.default_rng(n)
+    air = SynthTableAir(6, 8, 2)
+    desc = air.logup_descriptor()
+    desc["term_cols"] = np.array([0, 1, 2, 3], np.uint32)
+    main, al, z = rf(rng, (n, 8)), rf(rng, (air.max_alpha, 3)), rf(rng, (3,))
+    aux, total = mc.logup_aux_resident(main, desc, al, z, be)
+    want, wtotal = O.logup_aux(main, desc, al, z)
+    assert (np.asarray(total) == O.canon_array(np.asarray(wtotal, np.uint64).reshape(-1))).all()
+    assert (aux.reshape(-1) == O.canon_array(np.asarray(want, np.uint64).reshape(-1))).all()
