@@ -213,6 +213,12 @@ inline int check_launch(Ctx* ctx, const char* what) {
     return check_fault(ctx);
 }
 
+// Sponges up to which two lanes hash one (kc::permute_pair): 2^13 pairs are
+// one warp on almost every scheduler of 148 SMs (512 of 592). Twice as many
+// are two warps a scheduler, as slow as one thread a sponge (both bound by ALU
+// issue).
+constexpr uint64_t KECCAK_PAIR_MAX = 1ULL << 13;
+
 // ---- internal kernel drivers (ntt.cu, merkle.cu) ----
 enum Dir { FWD = 0, INV = 1 };
 // Batched natural-order DFT over the rows of a row-major n x m matrix.

@@ -97,6 +97,69 @@ __device__ __forceinline__ void permute(uint64_t s[25]) {
     }
 }
 
+// One permutation by a pair of adjacent lanes of a warp: lane h of the pair
+// (h = lane & 1) holds the low (0) or high (1) 32-bit half of all 25 state
+// lanes. Theta and chi work on the halves separately; a 64-bit rotation takes
+// the partner's half by a shuffle. A warp alone on its scheduler issues one
+// ALU instruction every two cycles, so a permutation's time is its ALU count:
+// 90 a round here against 180 in one thread (4.6 us a permutation), with 29
+// shuffles beside them on another pipe. Used where there are too few sponges
+// to fill the schedulers; all 32 lanes of the warp must call it.
+template <int R>
+__device__ __forceinline__ uint32_t rot_half(uint32_t own) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 1);
+    if constexpr (R < 32)
+        return __funnelshift_l(other, own, R);
+    else
+        return __funnelshift_l(own, other, R - 32);
+}
+__device__ __forceinline__ void permute_pair(uint32_t s[25], uint32_t h) {
+#pragma unroll 1
+    for (int round = 0; round < 24; ++round) {
+        uint32_t C[5], R[5];
+#pragma unroll
+        for (int x = 0; x < 5; ++x) C[x] = s[x] ^ s[x + 5] ^ s[x + 10] ^ s[x + 15] ^ s[x + 20];
+#pragma unroll
+        for (int x = 0; x < 5; ++x) R[x] = rot_half<1>(C[x]);
+#define D(x) C[((x) + 4) % 5] ^ R[((x) + 1) % 5]
+        uint32_t B[25];
+        B[0] = s[0] ^ D(0);
+        B[10] = rot_half<1>(s[1] ^ D(1));
+        B[20] = rot_half<62>(s[2] ^ D(2));
+        B[5] = rot_half<28>(s[3] ^ D(3));
+        B[15] = rot_half<27>(s[4] ^ D(4));
+        B[16] = rot_half<36>(s[5] ^ D(0));
+        B[1] = rot_half<44>(s[6] ^ D(1));
+        B[11] = rot_half<6>(s[7] ^ D(2));
+        B[21] = rot_half<55>(s[8] ^ D(3));
+        B[6] = rot_half<20>(s[9] ^ D(4));
+        B[7] = rot_half<3>(s[10] ^ D(0));
+        B[17] = rot_half<10>(s[11] ^ D(1));
+        B[2] = rot_half<43>(s[12] ^ D(2));
+        B[12] = rot_half<25>(s[13] ^ D(3));
+        B[22] = rot_half<39>(s[14] ^ D(4));
+        B[23] = rot_half<41>(s[15] ^ D(0));
+        B[8] = rot_half<45>(s[16] ^ D(1));
+        B[18] = rot_half<15>(s[17] ^ D(2));
+        B[3] = rot_half<21>(s[18] ^ D(3));
+        B[13] = rot_half<8>(s[19] ^ D(4));
+        B[14] = rot_half<18>(s[20] ^ D(0));
+        B[24] = rot_half<2>(s[21] ^ D(1));
+        B[9] = rot_half<61>(s[22] ^ D(2));
+        B[19] = rot_half<56>(s[23] ^ D(3));
+        B[4] = rot_half<14>(s[24] ^ D(4));
+#undef D
+#pragma unroll
+        for (int y = 0; y < 5; ++y) {
+#pragma unroll
+            for (int x = 0; x < 5; ++x)
+                s[x + 5 * y] = B[x + 5 * y] ^ (~B[(x + 1) % 5 + 5 * y] & B[(x + 2) % 5 + 5 * y]);
+        }
+        const uint64_t rc = RC[round];
+        s[0] ^= h ? (uint32_t)(rc >> 32) : (uint32_t)rc;
+    }
+}
+
 __device__ __forceinline__ uint64_t bswap64(uint64_t x) {
     uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32);
     return ((uint64_t)__byte_perm(lo, 0, 0x0123) << 32) | __byte_perm(hi, 0, 0x0123);

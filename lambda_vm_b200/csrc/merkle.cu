@@ -14,7 +14,8 @@
 //
 // One thread owns one sponge: Keccak is a serial chain of permutations, and
 // with the state in registers the kernels are bound by INT issue, not HBM.
-// The tree kernel reduces 8 levels per launch inside shared memory.
+// Where there are too few sponges for that (a tree's top 14 levels, leaves of
+// small tables), two lanes share one: latency, not issue, is the bound there.
 #include "common.cuh"
 #include "gl.cuh"
 #include "keccak.cuh"
@@ -66,6 +67,56 @@ __global__ void __launch_bounds__(128) k_leaves(const uint64_t* __restrict__ dat
     o[1] = s[1];
     o[2] = s[2];
     o[3] = s[3];
+}
+
+// The same leaves with two lanes a sponge (kc::permute_pair), for tables with
+// too few leaves to give every scheduler a full warp (KECCAK_PAIR_MAX).
+template <bool LE>
+__global__ void __launch_bounds__(128) k_leaves_pair(const uint64_t* __restrict__ data, uint64_t row_u64, uint64_t c0,
+                                                     uint64_t w, uint32_t R, uint32_t log_rows, uint64_t num_leaves,
+                                                     uint32_t* __restrict__ out) {
+    const uint64_t id = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 1;
+    const uint32_t h = threadIdx.x & 1;
+    const uint64_t leaf = id < num_leaves ? id : num_leaves - 1;  // whole warps hash: the rest repeat the last leaf
+    auto row_of = [&](uint64_t r) -> const uint64_t* {
+        const uint64_t br = log_rows ? (__brevll(r) >> (64 - log_rows)) : 0;
+        return data + br * row_u64 + c0;
+    };
+    uint32_t s[25];
+#pragma unroll
+    for (int i = 0; i < 25; ++i) s[i] = 0;
+    const uint64_t total = (uint64_t)R * w;
+    const uint64_t* row = row_of(leaf * R);
+    uint32_t k = 0;
+    uint64_t c = 0;
+    auto next = [&]() -> uint32_t {
+        uint64_t v = gl::canon(__ldg(row + c));
+        if (++c == w) {
+            c = 0;
+            ++k;
+            if (k < R) row = row_of(leaf * R + k);
+        }
+        if (!LE) v = kc::bswap64(v);
+        return h ? (uint32_t)(v >> 32) : (uint32_t)v;
+    };
+    const uint64_t full = total / 17;
+    const uint32_t rem = (uint32_t)(total % 17);
+    for (uint64_t b = 0; b < full; ++b) {
+#pragma unroll
+        for (int i = 0; i < 17; ++i) s[i] ^= next();
+        kc::permute_pair(s, h);
+    }
+#pragma unroll
+    for (int i = 0; i < 17; ++i) {
+        if ((uint32_t)i < rem) s[i] ^= next();
+        if ((uint32_t)i == rem && h == 0) s[i] ^= 1u;
+    }
+    if (h) s[16] ^= 0x80000000u;
+    kc::permute_pair(s, h);
+    if (id < num_leaves) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) out[leaf * 8 + 2 * i + h] = s[i];
+    }
 }
 
 // Per-row leaves absorbed one column window at a time, for commits whose
@@ -147,36 +198,45 @@ __device__ __forceinline__ void hash_pair(const uint64_t* l, const uint64_t* r, 
     for (int i = 0; i < 4; ++i) d[i] = s[i];
 }
 
+// Half h of the digest of two adjacent child digests (16 words from `c`).
+__device__ __forceinline__ void hash_pair_half(const uint32_t* c, uint32_t h, uint32_t d[4]) {
+    uint32_t s[25];
+#pragma unroll
+    for (int i = 0; i < 25; ++i) s[i] = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s[i] = c[2 * i + h];
+    if (h)
+        s[16] = 0x80000000u;
+    else
+        s[8] = 1u;
+    kc::permute_pair(s, h);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] = s[i];
+}
+
 // Reduce `levels` tree levels above child level jc (2^jc nodes, starting at
-// node index 2^jc - 1). CTA b owns children [b*2^levels, (b+1)*2^levels).
-__global__ void __launch_bounds__(128) k_merkle_levels(uint64_t* nodes, uint32_t jc, uint32_t levels) {
-    __shared__ uint64_t sh[128 * 4];
-    const uint32_t t = threadIdx.x;
+// node index 2^jc - 1). CTA b owns children [b*2^levels, (b+1)*2^levels), two
+// lanes a parent (these levels are narrow: their time is the latency of a
+// permutation). Whole warps hash; lanes past the last parent repeat the first.
+__global__ void __launch_bounds__(128) k_merkle_levels(uint32_t* nodes, uint32_t jc, uint32_t levels) {
+    __shared__ uint32_t sh[2][64 * 8];
+    const uint32_t t = threadIdx.x >> 1, h = threadIdx.x & 1;
     const uint64_t b = blockIdx.x;
     uint32_t active = 1u << (levels - 1);
-    uint64_t d[4];
-    if (t < active) {
-        const uint64_t child = ((1ULL << jc) - 1) + (b << levels) + 2 * t;
-        hash_pair(nodes + child * 4, nodes + (child + 1) * 4, d);
-        const uint64_t parent = ((1ULL << (jc - 1)) - 1) + (b << (levels - 1)) + t;
+    for (uint32_t lvl = 0; lvl < levels; ++lvl, active >>= 1) {
+        const uint32_t* from = lvl ? sh[lvl & 1] + 16 * (t < active ? t : 0)
+                                   : nodes + (((1ULL << jc) - 1) + (b << levels) + 2 * (t < active ? t : 0)) * 8;
+        if ((threadIdx.x & ~31u) < 2 * active) {  // warp-uniform
+            uint32_t d[4];
+            hash_pair_half(from, h, d);
+            if (t < active) {
+                const uint32_t j = jc - 1 - lvl;
+                const uint64_t parent = ((1ULL << j) - 1) + (b << (levels - 1 - lvl)) + t;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            nodes[parent * 4 + i] = d[i];
-            sh[t * 4 + i] = d[i];
-        }
-    }
-    __syncthreads();
-    for (uint32_t lvl = 1; lvl < levels; ++lvl) {
-        active >>= 1;
-        if (t < active) hash_pair(sh + 8 * t, sh + 8 * t + 4, d);
-        __syncthreads();
-        if (t < active) {
-            const uint32_t j = jc - 1 - lvl;
-            const uint64_t parent = ((1ULL << j) - 1) + (b << (levels - 1 - lvl)) + t;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                nodes[parent * 4 + i] = d[i];
-                sh[t * 4 + i] = d[i];
+                for (int i = 0; i < 4; ++i) {
+                    nodes[parent * 8 + 2 * i + h] = d[i];
+                    sh[(lvl + 1) & 1][t * 8 + 2 * i + h] = d[i];
+                }
             }
         }
         __syncthreads();
@@ -208,6 +268,16 @@ int leaves_row_major(Ctx* ctx, cudaStream_t st, const uint64_t* data, uint64_t n
     SG_CHECK_ARG(col_start < col_end && col_end <= row_u64, "column range");
     SG_CHECK_ARG(((uintptr_t)out & 7) == 0, "leaf output must be 8-byte aligned");
     const uint64_t nl = num_rows / rows_per_leaf;
+    if (nl <= KECCAK_PAIR_MAX) {
+        const unsigned pg = (unsigned)((2 * nl + 127) / 128);
+        if (little_endian)
+            k_leaves_pair<true><<<pg, 128, 0, st>>>(data, row_u64, col_start, col_end - col_start, rows_per_leaf, lr,
+                                                    nl, (uint32_t*)out);
+        else
+            k_leaves_pair<false><<<pg, 128, 0, st>>>(data, row_u64, col_start, col_end - col_start, rows_per_leaf, lr,
+                                                     nl, (uint32_t*)out);
+        return check_launch(ctx, "k_leaves_pair");
+    }
     const unsigned grid = (unsigned)((nl + 127) / 128);
     if (little_endian)
         k_leaves<true><<<grid, 128, 0, st>>>(data, row_u64, col_start, col_end - col_start, rows_per_leaf, lr, nl,
@@ -223,17 +293,20 @@ int merkle_inner(Ctx* ctx, cudaStream_t st, uint8_t* nodes, uint64_t L) {
     SG_CHECK_ARG(lg >= 0, "leaf count must be a power of two");
     SG_CHECK_ARG(((uintptr_t)nodes & 7) == 0, "node buffer must be 8-byte aligned");
     uint32_t jc = (uint32_t)lg;
-    // Levels with at least 2^14 parents: one full-width launch per level.
+    // Levels with more than KECCAK_PAIR_MAX parents: one full-width launch per level.
     while (jc > 14) {
         const uint64_t parents = 1ULL << (jc - 1);
         k_merkle_level<<<(unsigned)((parents + 127) / 128), 128, 0, st>>>((uint64_t*)nodes, jc);
         SG_TRY(check_launch(ctx, "k_merkle_level"));
         --jc;
     }
+    // Then 128 CTAs (a warp on each scheduler of most SMs) down to 128 nodes,
+    // and one CTA to the root.
     while (jc > 0) {
-        const uint32_t levels = jc < 8 ? jc : 8;
+        const uint32_t levels = jc > 7 ? jc - 7 : jc;
         const uint64_t ctas = 1ULL << (jc - levels);
-        k_merkle_levels<<<(unsigned)ctas, 1u << (levels - 1), 0, st>>>((uint64_t*)nodes, jc, levels);
+        const unsigned threads = std::max(32u, 2u << (levels - 1));
+        k_merkle_levels<<<(unsigned)ctas, threads, 0, st>>>((uint32_t*)nodes, jc, levels);
         SG_TRY(check_launch(ctx, "k_merkle_levels"));
         jc -= levels;
     }

@@ -223,8 +223,8 @@ __global__ void __launch_bounds__(256) k_inv_denoms(const uint64_t* __restrict__
     }
 }
 
-// out_partial[(chunk * K + k) * cols + c] = sum over the chunk's rows i of
 // ---------------------------------------------------------------- barycentric sums
+// out_partial[(chunk * K + k) * cols + c] = sum over the chunk's rows i of
 //   points[i] * col_c(row i*stride) * inv_denoms[k][i]
 #define BARY_MAX_K 8
 #define BARY_PF 4  // rows in flight per thread: 4, 8, 16 measured 1.60, 1.79, 1.78 ms (2^20 x 256, K = 2)
@@ -486,6 +486,59 @@ __global__ void __launch_bounds__(128) k_fri_fold(const uint64_t* in, uint64_t h
             for (int q = 0; q < 4; ++q) leaves[4 * t + q] = s[q];
         }
     }
+}
+
+// The same fold for layers with few leaves: a lane per output, and the two
+// lanes of a leaf hash it together (kc::permute_pair). Whole warps run; lanes
+// past the end repeat the last pair.
+__global__ void __launch_bounds__(128) k_fri_fold_pair(const uint64_t* in, uint64_t h, const uint64_t* tw, uint64_t z0,
+                                                       uint64_t z1, uint64_t z2, const uint64_t* dz, uint64_t* out,
+                                                       uint64_t* tw_next, uint32_t* leaves) {
+    const uint64_t id = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t half = threadIdx.x & 1;
+    const uint64_t j = id < h ? id : h - 2 + half;
+    const fe3 zeta = dz ? fe3{dz[0], dz[1], dz[2]} : fe3{z0, z1, z2};
+    const uint64_t t = tw[j];
+    const fe3 a = gl::canon3(fold_one(in, j, t, zeta));
+    if (id < h) {
+        st3(out + 3 * j, a);
+        if (!half && tw_next) tw_next[j >> 1] = gl::canon(gl::sqr(t));
+    }
+    uint32_t s[25];
+#pragma unroll
+    for (int q = 0; q < 25; ++q) s[q] = 0;
+    const uint64_t c[3] = {kc::bswap64(a.c0), kc::bswap64(a.c1), kc::bswap64(a.c2)};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const uint32_t lo = (uint32_t)c[q], hi = (uint32_t)(c[q] >> 32);
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, half ? lo : hi, 1);  // the half the partner holds
+        s[q] = half ? got : lo;
+        s[3 + q] = half ? hi : got;
+    }
+    if (half)
+        s[16] = 0x80000000u;
+    else
+        s[6] = 1u;
+    kc::permute_pair(s, half);
+    if (id < h) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) leaves[8 * (j >> 1) + 2 * q + half] = s[q];
+    }
+}
+
+static int fri_fold_launch(Ctx* ctx, cudaStream_t st, const uint64_t* in, uint64_t h, const uint64_t* tw,
+                           const uint64_t* zeta, const uint64_t* dz, uint64_t* out, uint64_t* tw_next,
+                           uint8_t* leaves) {
+    const uint64_t z[3] = {zeta ? zeta[0] : 0, zeta ? zeta[1] : 0, zeta ? zeta[2] : 0};
+    if (leaves && h <= 2 * KECCAK_PAIR_MAX) {
+        k_fri_fold_pair<<<(unsigned)((h + 127) / 128), 128, 0, st>>>(in, h, tw, z[0], z[1], z[2], dz, out, tw_next,
+                                                                     (uint32_t*)leaves);
+        return check_launch(ctx, "k_fri_fold_pair");
+    }
+    const uint64_t threads = (h + 1) / 2;
+    k_fri_fold<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(in, h, tw, z[0], z[1], z[2], dz, out, tw_next,
+                                                                  (uint64_t*)leaves);
+    return check_launch(ctx, "k_fri_fold");
 }
 
 // Leaves of an already-folded layer (pairs of consecutive ext3 values).
@@ -846,10 +899,8 @@ int sg_fri_fold_layer(sg_ctx* c, void* stream, const uint64_t* d_in, uint64_t h,
     SG_ENTER(ctx_of(c));
     SG_CHECK_ARG(!d_leaves || (h % 2 == 0), "leaves need an even folded length");
     if (h == 0) return SG_OK;
-    const uint64_t threads = (h + 1) / 2;
-    k_fri_fold<<<(unsigned)((threads + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
-        d_in, h, d_inv_tw, zeta[0], zeta[1], zeta[2], nullptr, d_out, d_inv_tw_next, (uint64_t*)d_leaves);
-    return check_launch(CX(c), "k_fri_fold");
+    return fri_fold_launch(CX(c), (cudaStream_t)stream, d_in, h, d_inv_tw, zeta, nullptr, d_out, d_inv_tw_next,
+                           d_leaves);
 }
 
 int sg_fri_leaves(sg_ctx* c, void* stream, const uint64_t* d_evals, uint64_t n, uint8_t* d_leaves) {
@@ -1228,10 +1279,7 @@ int fri_challenge_dev(Ctx* ctx, cudaStream_t st, void* d_state, const uint8_t* d
 int fri_fold_dev(Ctx* ctx, cudaStream_t st, const uint64_t* d_in, uint64_t h, const uint64_t* d_inv_tw,
                  const uint64_t* d_zeta, uint64_t* d_out, uint64_t* d_inv_tw_next, uint8_t* d_leaves) {
     if (h == 0) return SG_OK;
-    const uint64_t threads = (h + 1) / 2;
-    k_fri_fold<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(d_in, h, d_inv_tw, 0, 0, 0, d_zeta, d_out,
-                                                                  d_inv_tw_next, (uint64_t*)d_leaves);
-    return check_launch(ctx, "k_fri_fold");
+    return fri_fold_launch(ctx, st, d_in, h, d_inv_tw, nullptr, d_zeta, d_out, d_inv_tw_next, d_leaves);
 }
 
 }  // namespace sg

@@ -46,3 +46,37 @@ def test_logup_segments(be, n):
     want, wtotal = O.logup_aux(main, desc, al, z)
     assert (np.asarray(total) == O.canon_array(np.asarray(wtotal, np.uint64).reshape(-1))).all()
     assert (aux.reshape(-1) == O.canon_array(np.asarray(want, np.uint64).reshape(-1))).all()
+
+
+@pytest.mark.parametrize("h", [2, 6, 126, 130, 1 << 14, (1 << 14) + 2])
+def test_fri_fold_with_leaves(be, h):
+    rng = np.random.default_rng(h)
+    ev, tw, zeta = rf(rng, (6 * h,)), rf(rng, (h,)), rf(rng, (3,))
+    out, tn, lv = mc.fri_fold(ev, tw, zeta, True, be)
+    want = O.canon_array(O.fri_fold(ev, tw, zeta)).reshape(-1)
+    assert (out == want).all()
+    assert (tn == O.canon_array(np.array([O.gl_mul(int(t), int(t)) for t in tw[::2]], np.uint64))).all()
+    be_rows = want.reshape(-1, 6)
+    for q in {0, 1, h // 4, h // 2 - 1} & set(range(h // 2)):
+        assert bytes(lv[q]) == mc.keccak256(be_rows[q].astype(">u8").tobytes())
+
+
+@pytest.mark.parametrize("rows,cols,rpl,le", [(1 << 13, 9, 1, True), (1 << 14, 9, 1, True), (1 << 14, 35, 2, False),
+                                              (1 << 15, 35, 2, False), (64, 300, 2, False), (2, 17, 2, False),
+                                              (8, 34, 4, True)])
+def test_leaves_and_tree(be, rows, cols, rpl, le):
+    d = np.random.default_rng(rows + cols).integers(0, 2**64, size=(rows, cols), dtype=np.uint64)
+    got = mc.keccak_leaves_row_major(d, rpl, le, None, be)
+    want = O.leaves_row_major(d, rpl, le)
+    assert (got == np.asarray(want, np.uint8).reshape(got.shape)).all()
+    nodes = mc.build_merkle_tree_on_device(got, be)
+    assert bytes(nodes[0]) == O.merkle_root(want)
+    for q in {0, len(nodes) // 4, len(nodes) // 2 - 1} if len(nodes) > 1 else ():
+        assert bytes(nodes[q]) == mc.keccak256(bytes(nodes[2 * q + 1]) + bytes(nodes[2 * q + 2]))
+
+
+@pytest.mark.parametrize("lg", list(range(0, 17)))
+def test_tree_depths(be, lg):
+    leaves = np.random.default_rng(lg).integers(0, 256, size=(1 << lg, 32), dtype=np.uint8)
+    nodes = mc.build_merkle_tree_on_device(leaves, be)
+    assert bytes(nodes[0]) == O.merkle_root(leaves)
