@@ -234,15 +234,23 @@ static __global__ void k_shift_constraints(const uint64_t* __restrict__ cm, cons
         uint64_t sv[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) sv[k] = w.M(SH_S + k);
-        for (int j = 0; j < 64; ++j) {
-            gl::wacc lo = gl::wzero(), hi = gl::wzero();
+        // four bits at a time, their 18 operand bits read once into registers
+        // (16 reads a bit, two per product, were what bound this kernel)
+        for (int j0 = 0; j0 < 64; j0 += 4) {
+            uint64_t ab[18];  // a[j0 - 7 .. j0 + 10]
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (j - k >= 0) gl::wmac(lo, sv[k], w.M(SH_AB + j - k));
-                if (j + k < 64) gl::wmac(hi, sv[k], w.M(SH_AB + j + k));
+            for (int i = 0; i < 18; ++i) ab[i] = (unsigned)(j0 + i - 7) < 64u ? w.M(SH_AB + j0 + i - 7) : 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                gl::wacc lo = gl::wzero(), hi = gl::wzero();
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    gl::wmac(lo, sv[k], ab[7 + i - k]);
+                    gl::wmac(hi, sv[k], ab[7 + i + k]);
+                }
+                const uint64_t t = gl::add(gl::mul(nd, gl::wreduce(lo)), gl::mul(d, gl::wreduce(hi)));
+                s.put(gl::sub(w.M(SH_TB + j0 + i), t));
             }
-            const uint64_t t = gl::add(gl::mul(nd, gl::wreduce(lo)), gl::mul(d, gl::wreduce(hi)));
-            s.put(gl::sub(w.M(SH_TB + j), t));
         }
         // the result moves TB by whole bytes: byte k = sum_q Q_q (nd tB[k - q] + d tB[k + q])
         uint64_t tB[8];
