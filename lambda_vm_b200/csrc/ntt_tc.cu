@@ -57,8 +57,11 @@
 #include "common.cuh"
 #include "dft.cuh"
 #include "gl.cuh"
+#include "tc.cuh"
 
 namespace sg {
+
+using namespace tc;
 
 namespace {
 
@@ -86,64 +89,6 @@ struct TcPlan {
     static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// One bounded look at the barrier's phase: the thread sleeps until it
-// completes, or for the hinted time (ns).
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(100000u)
-        : "memory");
-    return ok != 0;
-}
-__device__ __noinline__ void mbar_wait_slow(uint32_t bar, uint32_t parity, volatile uint32_t* abort, unsigned* err) {
-    uint64_t t0, t1;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    do {
-        for (int i = 0; i < 64; ++i)
-            if (mbar_try(bar, parity)) return;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-    } while (!*abort && t1 - t0 < 2000000000ull);
-    *abort = 1;
-    *(volatile unsigned*)err = 1;
-}
-// Wait for the barrier's phase, two seconds at most; on a timeout the CTA's
-// abort word is set (every later wait then returns at once and the CTA leaves
-// the kernel at its next tile) and so is the context's error word.
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort, unsigned* err) {
-    if (!mbar_try(bar, parity)) mbar_wait_slow(bar, parity, abort, err);
-}
-
-// K-major operand without swizzle: 8 x 16-byte core matrices of 128 contiguous
-// bytes; lbo: bytes between the two 16-byte K slices, sbo: between 8-row groups.
-__device__ __forceinline__ uint64_t mma_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
-           (1ull << 46);
-}
-// u8 x u8 -> s32, M = 128, N columns
-__host__ __device__ constexpr uint32_t mma_idesc(uint32_t n) { return (2u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
-
-// One thread of a warp (the branch it guards is warp-uniform, so the
-// descriptors stay in uniform registers).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok));
-    return ok != 0;
-}
-
 // One step's products: MT accumulators of 128 x N s32 side by side from TMEM
 // column d on = A (128 rows each, A_TILE bytes apart) x B (N rows)^T over
 // KS K steps of 32 bytes, then an arrive on `bar` when they have completed.
@@ -157,14 +102,9 @@ __device__ __forceinline__ void mma_step(uint32_t d, uint32_t a, uint32_t b, uin
             const uint64_t da = mma_desc(a + t * A_TILE, A_LBO, 128);
 #pragma unroll
             for (uint32_t k = 0; k < KS; ++k)
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d + t * N),
-                    "l"(da + k * ((2 * A_LBO) >> 4)), "l"(db + k * ((2 * B_LBO) >> 4)), "r"(mma_idesc(N)), "r"(k)
-                    : "memory");
+                mma_i8(d + t * N, da + k * ((2 * A_LBO) >> 4), db + k * ((2 * B_LBO) >> 4), N, k);
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+        mma_commit(bar);
     }
     __syncwarp();
 }
@@ -212,24 +152,11 @@ __device__ __forceinline__ uint64_t recombine(const uint32_t* v) {
     return gl::reduce96(w0, w1, w2);
 }
 
-__device__ __forceinline__ void sts128(uint32_t addr, uint64_t x, uint64_t y) {
-    asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(addr), "l"(x), "l"(y) : "memory");
-}
 // 8 bytes from global to shared memory without registers; zeros when !valid.
 __device__ __forceinline__ void copy_async8(uint32_t dst, const uint64_t* src, bool valid) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-// Arrive on the barrier when this thread's copies so far have landed.
-__device__ __forceinline__ void copy_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
 // Barrier of the 512 working threads; the OR of their predicates.
 __device__ __forceinline__ bool bar_or(bool x) {
     uint32_t ok;
@@ -244,10 +171,6 @@ __device__ __forceinline__ bool bar_or(bool x) {
     return ok != 0;
 }
 __device__ __forceinline__ void bar_all() { asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); }
-__device__ __forceinline__ void sts64(uint32_t addr, uint64_t x) {
-    asm volatile("st.shared.u64 [%0], %1;" ::"r"(addr), "l"(x) : "memory");
-}
-
 // The byte matrix of an R-point DFT over coset `shift` of 2^lb:
 // c(k, j, b) = w_R^{+-jk} w_{2^lb R}^{shift j} 2^8b, at row 8 k + d, K byte
 // 8 j + b in the core-matrix layout (K slice stride 128 R bytes).

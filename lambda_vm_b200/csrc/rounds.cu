@@ -17,6 +17,7 @@
 #include "gl.cuh"
 #include "keccak.cuh"
 #include "fs.cuh"
+#include "tc.cuh"
 
 namespace sg {
 
@@ -329,6 +330,173 @@ static bary_fn bary_kernel(uint32_t K) {
         case 7: return k_bary<EXT3, 7>;
         default: return k_bary<EXT3, 8>;
     }
+}
+
+// The sums over base-field columns as byte products on the tensor cores. With
+// t = sum_b t_b 2^8b and the weights W_q(i) = points[i] inv_denoms[k][i]
+// (q = (k, component)) in bytes a,
+//   S_q(c) = sum_{a,b} 2^8(a+b) sum_i W_q(i)_a t_i(c)_b,
+// the inner sums being one exact u8 x u8 -> s32 product over the rows: M =
+// (byte b, column c) of 16 columns, N = (q, a), K = rows. Both operands want
+// the rows' bytes side by side, so a thread takes 16 rows of one column,
+// transposes their bytes (64 byte permutes) and stores 16-byte pieces; the
+// products themselves are free. About 7 instructions a cell where k_bary's
+// multiply-accumulates take 54 at K = 2. A CTA takes a column tile of at most
+// 80 columns (five M-tiles, 240 TMEM columns) and a chunk of rows; two CTAs
+// share an SM, one loading while the other's products run. The accumulators
+// hold 2^31 / 255^2 > 32768 rows. 2^19 points x 200 columns (every second row),
+// two points: 811 us in k_bary, 291 here (2.9 TB/s).
+constexpr uint32_t BT_COLS = 80, BT_ROWS = 128, BT_MT = 5, BT_THREADS = 256;
+constexpr uint32_t BT_MAX_CHUNK = 32768;
+constexpr uint64_t BT_MIN_ROWS = 1ULL << 15, BT_MIN_COLS = 12;
+template <int K>
+struct BaryTc {
+    static constexpr uint32_t Q = 3 * K, N = K == 1 ? 32 : 48;  // N: a multiple of 16
+    static constexpr uint32_t A_TILE = 128 * BT_ROWS, W_LBO = N * 16;
+    static constexpr uint32_t OFF_W = BT_MT * A_TILE, OFF_BAR = OFF_W + N * BT_ROWS;
+    static constexpr uint32_t SMEM = OFF_BAR + 32;
+};
+
+// Bytes of four words, transposed: word j of the result holds byte j of each.
+__device__ __forceinline__ void transpose4(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t o[4]) {
+    const uint32_t t0 = __byte_perm(a, b, 0x5140), t1 = __byte_perm(c, d, 0x5140), t2 = __byte_perm(a, b, 0x7362),
+                   t3 = __byte_perm(c, d, 0x7362);
+    o[0] = __byte_perm(t0, t1, 0x5410), o[1] = __byte_perm(t0, t1, 0x7632);
+    o[2] = __byte_perm(t2, t3, 0x5410), o[3] = __byte_perm(t2, t3, 0x7632);
+}
+
+template <int K>
+__global__ void __launch_bounds__(BT_THREADS, 2)
+    k_bary_tc(const uint64_t* __restrict__ data, uint64_t row_u64, uint64_t stride, uint32_t cols, uint32_t CT,
+              const uint64_t* __restrict__ points, const uint64_t* __restrict__ invd, uint64_t n, uint64_t chunk_len,
+              uint64_t* __restrict__ partial, unsigned* err) {
+    using namespace tc;
+    using B = BaryTc<K>;
+    constexpr uint32_t Q = B::Q, N = B::N;
+    extern __shared__ __align__(1024) uint8_t bt_sm[];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid / 32, 0);
+    const uint32_t A = smem_addr(bt_sm), Wb = A + B::OFF_W, bar = A + B::OFF_BAR;
+    uint32_t* ctrl = reinterpret_cast<uint32_t*>(bt_sm + B::OFF_BAR + 8);  // TMEM address, abort word
+    volatile uint32_t* abort = ctrl + 1;
+    const uint32_t c0 = blockIdx.x * CT, ncols = min(CT, cols - c0), mt = (ncols + 15) / 16;
+    const uint64_t i0 = blockIdx.y * chunk_len, i1 = min(n, i0 + chunk_len);
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_addr(ctrl)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        *abort = 0;
+    }
+    // the weights' rows past (q, a) stay zero
+    if (K == 1)
+        for (uint32_t e = tid; e < N * BT_ROWS / 8; e += BT_THREADS) sts64(Wb + 8 * e, 0);
+    fence_async();
+    tc_before();
+    __syncthreads();
+    tc_after();
+    const uint32_t tmem = ctrl[0];
+    uint32_t turn = 0;
+    for (uint64_t r0 = i0; r0 < i1; r0 += BT_ROWS, ++turn) {
+        if (turn) mbar_wait(bar, (turn - 1) & 1, abort, err);  // the previous products have read A and W
+        // ---- columns: 16 rows of one column a turn
+        for (uint32_t e = tid; e < 16 * mt * (BT_ROWS / 16); e += BT_THREADS) {
+            const uint32_t c = e % (16 * mt), s = e / (16 * mt);
+            const uint64_t i = r0 + 16 * s;
+            const uint64_t* p = data + i * stride * row_u64 + c0 + c;
+            const uint64_t step = stride * row_u64;
+            uint64_t t[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) t[r] = c < ncols && i + r < i1 ? __ldg(p + r * step) : 0;
+            const uint32_t dst = A + (c >> 4) * B::A_TILE + s * 2048 + (c & 15) * 16;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t o[4][4];  // [row group][byte]
+#pragma unroll
+                for (int g = 0; g < 4; ++g)
+                    transpose4((uint32_t)(t[4 * g] >> (32 * half)), (uint32_t)(t[4 * g + 1] >> (32 * half)),
+                               (uint32_t)(t[4 * g + 2] >> (32 * half)), (uint32_t)(t[4 * g + 3] >> (32 * half)), o[g]);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    sts128(dst + (4 * half + b) * 256, gl::pack(o[0][b], o[1][b]), gl::pack(o[2][b], o[3][b]));
+            }
+        }
+        // ---- weights: four rows of one (k, component) a turn
+        for (uint32_t e = tid; e < Q * (BT_ROWS / 4); e += BT_THREADS) {
+            const uint32_t q = e / (BT_ROWS / 4), g = e % (BT_ROWS / 4);
+            uint64_t w[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const uint64_t i = r0 + 4 * g + r;
+                w[r] = i < i1 ? gl::mul(__ldg(invd + 3 * ((q / 3) * n + i) + q % 3), __ldg(points + i)) : 0;
+            }
+            const uint32_t dst = Wb + (g >> 2) * B::W_LBO + q * 128 + (g & 3) * 4;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t o[4];
+                transpose4((uint32_t)(w[0] >> (32 * half)), (uint32_t)(w[1] >> (32 * half)),
+                           (uint32_t)(w[2] >> (32 * half)), (uint32_t)(w[3] >> (32 * half)), o);
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (4 * half + b) * 16), "r"(o[b]) : "memory");
+            }
+        }
+        fence_async();
+        __syncthreads();
+        if (warp == 0) {
+            tc_after();
+            if (elect_one()) {
+                for (uint32_t m = 0; m < mt; ++m) {
+                    const uint64_t da = mma_desc(A + m * B::A_TILE, 2048, 128), db = mma_desc(Wb, B::W_LBO, 128);
+#pragma unroll
+                    for (uint32_t k = 0; k < BT_ROWS / 32; ++k)
+                        mma_i8(tmem + m * N, da + k * (4096 >> 4), db + k * ((2 * B::W_LBO) >> 4), N, turn + k);
+                }
+                mma_commit(bar);
+            }
+            __syncwarp();
+        }
+    }
+    if (turn) mbar_wait(bar, (turn - 1) & 1, abort, err);
+    tc_after();
+    // ---- accumulators: row (b, c), column (q, a); sum_a first, times 2^8b, then over b
+    uint64_t* red = reinterpret_cast<uint64_t*>(bt_sm);  // [M-tile][row][q]; the products are done with A
+    for (uint32_t m = warp >> 2; m < mt; m += 2) {
+        const uint32_t row = 32 * (warp & 3) + lane;
+        const uint64_t scale = 1ull << (8 * (row >> 4));
+#pragma unroll
+        for (uint32_t q = 0; q < Q; ++q) {
+            uint32_t v[8];
+            tmem_ld8(tmem + ((32u * (warp & 3)) << 16) + m * N + 8 * q, v);
+            // limbs below 2^31: two 56-bit halves
+            const uint64_t lo = v[0] + ((uint64_t)v[1] << 8) + ((uint64_t)v[2] << 16) + ((uint64_t)v[3] << 24);
+            const uint64_t hi = v[4] + ((uint64_t)v[5] << 8) + ((uint64_t)v[6] << 16) + ((uint64_t)v[7] << 24);
+            const uint64_t mid = (lo >> 32) + (uint32_t)hi;
+            const uint64_t x = gl::reduce96((uint32_t)lo, (uint32_t)mid, (uint32_t)((hi >> 32) + (mid >> 32)));
+            red[(m * 128 + row) * Q + q] = gl::mul(x, scale);
+        }
+    }
+    tc_before();
+    __syncthreads();
+    tc_after();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
+    for (uint32_t e = tid; e < ncols * Q; e += BT_THREADS) {
+        const uint32_t c = e / Q, q = e % Q;
+        uint64_t t = 0;
+        for (uint32_t b = 0; b < 8; ++b) t = gl::add(t, red[((c >> 4) * 128 + b * 16 + (c & 15)) * Q + q]);
+        partial[3 * ((blockIdx.y * (uint64_t)K + q / 3) * cols + c0 + c) + q % 3] = t;
+    }
+}
+
+template <int K>
+static int bary_tc_launch(Ctx* ctx, cudaStream_t st, const uint64_t* data, uint64_t row_u64, uint64_t stride,
+                          uint32_t cols, uint32_t CT, const uint64_t* points, const uint64_t* invd, uint64_t n,
+                          uint64_t chunk_len, uint64_t* part, dim3 grid) {
+    KernelInfo ki;
+    SG_TRY(kernel_info((const void*)k_bary_tc<K>, BaryTc<K>::SMEM, BT_THREADS, &ki));
+    k_bary_tc<K><<<grid, BT_THREADS, BaryTc<K>::SMEM, st>>>(data, row_u64, stride, cols, CT, points, invd, n, chunk_len,
+                                                            part, ctx->fault_dev);
+    return check_launch(ctx, "k_bary_tc");
 }
 
 // One warp per output: lanes sum strided chunk partials, then a shuffle tree.
@@ -781,6 +949,31 @@ int sg_barycentric_sums(sg_ctx* c, void* stream, const uint64_t* d_data, uint64_
         SG_CUDA(cudaMemsetAsync(d_out, 0, 24ull * k * cols, st));
         return SG_OK;
     }
+    auto combine = [&](uint64_t* part, uint64_t chunks) {
+        const uint64_t per = (uint64_t)k * cols;
+        k_bary_combine<<<(unsigned)((per * 32 + 255) / 256), 256, 0, st>>>(part, chunks, per, d_out);
+        return check_launch(ctx, "k_bary_combine");
+    };
+    // Base-field columns at one or two points over many rows: tensor cores
+    if (!ext3 && k <= 2 && n >= BT_MIN_ROWS && cols >= BT_MIN_COLS && cols < (1u << 24) && ctx->fault_dev) {
+        const uint64_t tiles = (cols + BT_COLS - 1) / BT_COLS, CT = (cols + tiles - 1) / tiles;
+        // two CTAs an SM in all; a chunk is whole turns and fits the accumulators
+        uint64_t len = (n * tiles + 295) / 296;
+        len = std::min<uint64_t>((len + BT_ROWS - 1) / BT_ROWS * BT_ROWS, BT_MAX_CHUNK);
+        const uint64_t chunks = (n + len - 1) / len;
+        if (chunks <= 65535) {
+            uint64_t* part = nullptr;
+            const uint64_t bytes = 24ull * chunks * k * cols;
+            SG_TRY(dev_alloc(ctx, st, bytes, (void**)&part));
+            const dim3 grid((unsigned)tiles, (unsigned)chunks);
+            int rc = (k == 1 ? bary_tc_launch<1> : bary_tc_launch<2>)(ctx, st, d_data, row_u64, row_stride, (uint32_t)cols,
+                                                                      (uint32_t)CT, d_points, d_inv_denoms, n, len,
+                                                                      part, grid);
+            if (rc == SG_OK) rc = combine(part, chunks);
+            const int rf = dev_free(ctx, st, part, bytes);
+            return rc != SG_OK ? rc : rf;
+        }
+    }
     // Column tile of at most 512 threads; row lanes fill the block to >= 256 threads.
     const uint64_t ctiles = (cols + 511) / 512;
     const uint32_t CT = (uint32_t)((cols + ctiles - 1) / ctiles);
@@ -804,11 +997,7 @@ int sg_barycentric_sums(sg_ctx* c, void* stream, const uint64_t* d_data, uint64_
     fn<<<grid, threads, smem, st>>>(d_data, row_u64, row_stride, cols, CT, RL, RB, d_points, d_inv_denoms, n, chunk_len,
                                     part);
     int rc = check_launch(ctx, "k_bary");
-    if (rc == SG_OK) {
-        const uint64_t per = (uint64_t)k * cols;
-        k_bary_combine<<<(unsigned)((per * 32 + 255) / 256), 256, 0, st>>>(part, chunks, per, d_out);
-        rc = check_launch(ctx, "k_bary_combine");
-    }
+    if (rc == SG_OK) rc = combine(part, chunks);
     int rf = dev_free(ctx, st, part, 24ull * chunks * k * cols);
     return rc != SG_OK ? rc : rf;
 }

@@ -34,6 +34,25 @@ def test_zero_denominator_is_reported(be):
         mc.compute_and_invert_denoms_ext3(x, np.array([[7, 1, 2], [4321, 0, 0]], np.uint64), 1, be)
 
 
+# From 2^15 rows and 12 base columns on, one or two points: column tiles of at
+# most 80 in groups of 16, turns of 128 rows, chunks of whole turns. Columns,
+# strides and rows that end inside each; bytes of 255 in every place.
+@pytest.mark.parametrize("n,ru,cols,stride,k", [(1 << 15, 12, 12, 1, 1), ((1 << 15) + 1, 20, 17, 2, 2),
+                                                ((1 << 15) + 127, 81, 80, 1, 2), (40000, 81, 81, 1, 1),
+                                                (100001, 170, 161, 1, 2), (1 << 17, 33, 33, 2, 2),
+                                                ((1 << 15) - 1, 16, 16, 1, 2), (1 << 15, 11, 11, 1, 2)])
+@pytest.mark.parametrize("ones", [False, True])
+def test_barycentric_sums_of_base_columns(be, n, ru, cols, stride, k, ones):
+    rng = np.random.default_rng(n + cols)
+    data = np.full((n * stride, ru), 2**64 - 1, np.uint64) if ones else rng.integers(0, 2**64, (n * stride, ru), np.uint64)
+    pts, invd = rf(rng, (n,)), rf(rng, (k * n * 3,))
+    if ones:
+        pts[:], invd[:] = 1, P - 2
+    got = mc.barycentric_multi(data, stride, False, cols, pts, invd, n, k, be)
+    want = O.canon_array(O.barycentric_sums(data, stride, False, cols, pts, invd, n, k))
+    assert (got == want).all()
+
+
 # 1024-row segments: one a scanning thread up to 2^20 rows, two and three above
 @pytest.mark.parametrize("n", [1, 1024, 1025, 1 << 20, (1 << 20) + 5, (1 << 21) + 1024])
 def test_logup_segments(be, n):
