@@ -761,9 +761,16 @@ int sg_eval_constraints(sg_ctx* c, void* stream, const sg_device_program* prog, 
                                                           comp ? 0 : 1, comp ? d_extra : d_out);
                 rc = check_launch(ctx, "k_shift_constraints");
             } else {
-                k_cpu_constraints<<<grid, 128, 0, st>>>(d_cm, d_main, m, rows, next_step, hand_chips,
-                                                        d_blob + o_beta, comp ? 0 : 1, comp ? d_extra : d_out);
-                rc = check_launch(ctx, "k_cpu_constraints");
+                KernelInfo ki;
+                const size_t sm = cpu_air_smem(CPU_FULL_WIDTH);  // of the widest set: one attribute for the kernel
+                rc = kernel_info((const void*)k_cpu_constraints, sm, CPU_WARPS * 32, &ki);
+                if (rc == SG_OK) {
+                    const uint64_t tiles = (rows + CPU_TILE - 1) / CPU_TILE, cap = (uint64_t)ki.sms * ki.blocks_per_sm;
+                    k_cpu_constraints<<<(unsigned)(tiles < cap ? tiles : cap), CPU_WARPS * 32, sm, st>>>(
+                        d_main, (uint32_t)m, rows, next_step, hand_chips, d_blob + o_beta, comp ? 0 : 1,
+                        comp ? d_extra : d_out);
+                    rc = check_launch(ctx, "k_cpu_constraints");
+                }
             }
         }
         if (rc == SG_OK && lg) {

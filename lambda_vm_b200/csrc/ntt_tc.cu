@@ -24,9 +24,9 @@
 //            rows, so M-tile m's outputs land exactly in the part of A that
 //            M-tile m was read from, and the exchange is in place.
 // A stage takes four steps of 256 TMEM columns (the products of one M-tile for
-// R = 32, two for R = 16, four for R = 8) in two accumulators. The warps meet only through
-// mbarriers (product complete, accumulator read, tile landed, stage 1's
-// outputs written), so the products run under the arithmetic and the warps
+// R = 32, two for R = 16, four for R = 8) in two accumulators. The warps meet
+// only through mbarriers (product complete, accumulator read, tile landed,
+// stage 1's outputs written), so the products run under the arithmetic and the warps
 // drift apart; the next tile's loads (8-byte asynchronous copies: the bytes
 // of a word stay together, the words of a row segment go to different rows)
 // start when stage 2's last product has completed, under its last two steps.
@@ -38,11 +38,12 @@
 // takes 14.3 ms, without its HBM accesses 14.1, with neither 8.6. The products
 // run at the tensor cores' full i8 rate (128 cycles per 128 x 256 x 32) and
 // take 4.6 ms of it; the arithmetic issues 64 cycles a warp for a stage-1
-// output. The HBM side is bound by address translation, not bytes (DRAM 20 %
-// busy): the rows of a four-step tile lie in different pages, so the bytes of
-// a row segment count. A 2^10-point tile takes 16 columns, 128 bytes; 8
-// columns (two independent groups of 256 threads) took 18.9 ms, and touching
-// the next tile's rows with L2 prefetches on top 37.7.
+// output. The HBM side is not bound by bytes (DRAM 20 % busy): a tile's 128 KB
+// are asked for in one burst, in its last two steps, as 128-byte row segments
+// (16 columns of a 2^10-point tile). 8 columns (two independent groups of 256
+// threads) took 18.9 ms, touching the next tile's rows with L2 prefetches on
+// top 37.7; scratch matrices in blocks of 16 columns, whole tiles of which are
+// contiguous, made no difference (18.35).
 //
 // Coset shifts cost nothing: a forward pass over coset `rep` multiplies input
 // i by w_{B L}^{i rep}; its j1 part goes into the constant matrix, the j2 part
@@ -50,7 +51,7 @@
 // therefore works on one rep (grid a multiple of reps), which also brings the
 // reps' reads of one input tile together in L2.
 //
-// Bound: integer issue and address translation, about equally (110 thread
+// Bound: integer issue and the tile loads' bursts, about equally (110 thread
 // instructions a point and pass where k_dft takes 180-230).
 #include <type_traits>
 
@@ -152,11 +153,6 @@ __device__ __forceinline__ uint64_t recombine(const uint32_t* v) {
     return gl::reduce96(w0, w1, w2);
 }
 
-// 8 bytes from global to shared memory without registers; zeros when !valid.
-__device__ __forceinline__ void copy_async8(uint32_t dst, const uint64_t* src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Barrier of the 512 working threads; the OR of their predicates.
 __device__ __forceinline__ bool bar_or(bool x) {
     uint32_t ok;
@@ -203,7 +199,7 @@ __global__ void __launch_bounds__(NT + 32, 1)
     k_dft_tc(PassArgs a, uint32_t gtiles, uint32_t ctiles, uint64_t flat_total, uint32_t lb, unsigned* err) {
     using PL = TcPlan<LR1, LR2, DBL, FLAT>;
     constexpr uint32_t R1 = PL::R1, R2 = PL::R2, T = PL::T, S = PL::S, D = PL::D, CSL = PL::CSL;
-    constexpr uint32_t ROWS1 = PTS / R1, ROWS2 = PTS / R2;  // instances of each stage
+    constexpr uint32_t ROWS2 = PTS / R2;  // instances of each stage
     constexpr uint32_t A_WORDS = FLAT ? CSL * R1 : R1;      // factor words a; b follows
     extern __shared__ __align__(1024) uint8_t sm8[];
     const uint32_t tid = threadIdx.x, lane = tid % 32;

@@ -1,5 +1,5 @@
-// tcgen05, TMEM and mbarrier primitives of the kernels that run byte products
-// (kind::i8, u8 x u8 -> s32) on the tensor cores.
+// Asynchronous copies, and the tcgen05, TMEM and mbarrier primitives of the
+// kernels that run byte products (kind::i8, u8 x u8 -> s32) on the tensor cores.
 #pragma once
 #include <stdint.h>
 
@@ -89,6 +89,11 @@ __device__ __forceinline__ bool elect_one() {
     return ok != 0;
 }
 
+// 8 bytes from global to shared memory without registers; zeros when !valid.
+__device__ __forceinline__ void copy_async8(uint32_t dst, const uint64_t* src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // Arrive on the barrier when this thread's copies so far have landed.
 __device__ __forceinline__ void copy_async_arrive(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");

@@ -1,12 +1,14 @@
 """Sizes at which the round kernels change form, against the CPU oracle: runs
 of 16 or 4 denominators a thread, more LogUp segments than scanning threads,
-two lanes or one thread a sponge (FRI layers, leaves, tree levels)."""
+two lanes or one thread a sponge (FRI layers, leaves, tree levels), tensor-core
+barycentric sums, tiles of the hand-written tables."""
 import numpy as np
 import pytest
 
 import oracle as O
-from lambda_vm_b200 import math_cuda as mc
+from lambda_vm_b200 import math_cuda as mc, rv64, rv64_air as RA
 from lambda_vm_b200.air import SynthTableAir
+from lambda_vm_b200.ir import lower
 
 pytestmark = pytest.mark.gpu
 P = O.P
@@ -99,3 +101,25 @@ def test_tree_depths(be, lg):
     leaves = np.random.default_rng(lg).integers(0, 256, size=(1 << lg, 32), dtype=np.uint8)
     nodes = mc.build_merkle_tree_on_device(leaves, be)
     assert bytes(nodes[0]) == O.merkle_root(leaves)
+
+
+# Tiles of 32 rows of the CPU table and windows of four bits of SHIFT: fewer rows
+# than a tile, rows that end inside one, a next row that wraps.
+@pytest.mark.parametrize("table", ["core", "all", "shift"])
+@pytest.mark.parametrize("rows,step", [(1, 0), (2, 1), (31, 1), (33, 2), (97, 4), (64, 2), (16, 2)])
+def test_table_kernels_at_tile_edges(be, table, rows, step):
+    rng = np.random.default_rng(rows)
+    if table == "shift":
+        air = RA.ShiftAir(8)
+    else:
+        air = RA.CpuAir(rv64.keccak_program(136), 9, ("bitwise", "shift", "memory", "keccak") if table == "all" else ())
+    full, dev = lower(air.program), lower(air.device_program)
+    main, aux = rf(rng, (rows, air.width)), rf(rng, (rows, 3 * air.aux_width))
+    rest = rf(rng, (2, 3)), rf(rng, (air.max_alpha, 3)), rf(rng, (3,)), step
+    comps = [None]
+    if rows >= 16 and rows & (rows - 1) == 0:
+        comps.append({"beta": rf(rng, (len(full["roots"]), 3)), "z_inv": rf(rng, (rows // 4,)),
+                      "boundary": [(air.acc_col, True, rf(rng, (3,)), rf(rng, (3,)))], "b_z_inv": rf(rng, (1, rows))})
+    for comp in comps:
+        want = mc.eval_constraints_on_device(full, main, aux, *rest, comp, be)
+        assert np.array_equal(mc.eval_constraints_on_device(dev, main, aux, *rest, comp, be), want)
