@@ -18,6 +18,10 @@
  *  - Matrices are row-major: element (row r, column c) at [r * row_stride + c].
  *  - Device pointers are named d_*; host pointers have no prefix.
  *  - One context per GPU; a context is safe to use from several threads.
+ *  - Kernels that wait for the tensor cores give up after two seconds. Results
+ *    of the context are then not to be trusted: the call that waits for them
+ *    (sg_stream_sync included), and every call after it that launches or waits,
+ *    returns SG_ERR_CUDA. This lasts; destroy the context and create another.
  */
 #ifndef STARKGPU_H
 #define STARKGPU_H
@@ -77,6 +81,10 @@ SG_API uint64_t sg_ctx_launches(sg_ctx* ctx);
 /* Test hook for host-side failure handling: the n-th device allocation from
  * now (n >= 1) fails with SG_ERR_OOM; n = 0 disarms. */
 SG_API int sg_ctx_fail_alloc_after(sg_ctx* ctx, int64_t n);
+/* Test hook for the tensor-core waits: the n-th kernel launch from now
+ * (n >= 1) leaves the context as a kernel that gave up its wait leaves it;
+ * n = 0 disarms. */
+SG_API int sg_ctx_fail_wait_after(sg_ctx* ctx, int64_t n);
 
 /* Stream-ordered device memory charged to the context budget. */
 SG_API int sg_dev_alloc(sg_ctx* ctx, void* stream, uint64_t bytes, void** d_out);

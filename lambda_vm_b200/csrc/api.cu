@@ -253,6 +253,13 @@ int sg_ctx_fail_alloc_after(sg_ctx* c, int64_t n) {
     return SG_OK;
 }
 
+int sg_ctx_fail_wait_after(sg_ctx* c, int64_t n) {
+    SG_CHECK_ARG(c && n >= 0, "bad argument");
+    SG_ENTER(ctx_of(c));
+    C(c)->fail_wait_after.store(n == 0 ? -1 : n);
+    return SG_OK;
+}
+
 int sg_dev_alloc(sg_ctx* c, void* stream, uint64_t bytes, void** d_out) {
     SG_CHECK_ARG(c && d_out, "null argument");
     SG_ENTER(ctx_of(c));
@@ -284,8 +291,7 @@ int sg_memcpy_d2h(sg_ctx* c, void* stream, void* dst, const void* src, uint64_t 
 int sg_stream_sync(sg_ctx* c, void* stream) {
     SG_CHECK_ARG(c, "null context");
     SG_ENTER(ctx_of(c));
-    SG_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-    return check_fault(C(c));
+    return sync_checked(C(c), (cudaStream_t)stream, "stream sync");
 }
 
 int sg_stream_create(sg_ctx* c, void** out) {
@@ -397,7 +403,7 @@ int sg_merkle_build(sg_ctx* c, void* stream, const uint8_t* d_leaves, uint64_t n
     SG_TRY(merkle_inner(C(c), st, d_nodes, L));
     if (root_out) {
         SG_CUDA(cudaMemcpyAsync(root_out, d_nodes, 32, cudaMemcpyDeviceToHost, st));
-        SG_CUDA(cudaStreamSynchronize(st));
+        SG_TRY(sync_checked(C(c), st, "merkle build"));
     }
     return SG_OK;
 }
@@ -678,11 +684,15 @@ int sg_lde_commit(sg_ctx* c, void* stream, const uint64_t* trace, int trace_on_d
     sg_lde* h = nullptr;
     SG_TRY(commit_enqueue(ctx, st, trace, trace_on_device, n, row_u64, blowup, weights, 0, layout, host_lde_out, &h));
     cudaError_t e = cudaMemcpyAsync(h->root, h->d_nodes, 32, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    int rc = SG_OK;
     if (e != cudaSuccess) {
         set_error(std::string("lde commit: ") + cudaGetErrorString(e));
+        rc = SG_ERR_CUDA;
+    }
+    if (rc == SG_OK) rc = sync_checked(ctx, st, "lde commit");
+    if (rc != SG_OK) {
         sg_lde_free(c, h);
-        return SG_ERR_CUDA;
+        return rc;
     }
     if (root_out) memcpy(root_out, h->root, 32);
     *out = h;
@@ -713,11 +723,11 @@ int sg_lde_commit_split(sg_ctx* c, void* stream, const uint64_t* trace, int trac
     uint8_t pre[32];
     cudaError_t e = rc == SG_OK ? cudaMemcpyAsync(h->root, h->d_nodes, 32, cudaMemcpyDeviceToHost, st) : cudaSuccess;
     if (rc == SG_OK && e == cudaSuccess && build_pre) e = cudaMemcpyAsync(pre, d_pre_nodes, 32, cudaMemcpyDeviceToHost, st);
-    if (rc == SG_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (rc == SG_OK && e != cudaSuccess) {
         set_error(std::string("lde commit split: ") + cudaGetErrorString(e));
         rc = SG_ERR_CUDA;
     }
+    if (rc == SG_OK) rc = sync_checked(ctx, st, "lde commit split");
     if (rc != SG_OK) {
         sg_lde_free(c, h);
         return rc;
@@ -791,7 +801,8 @@ int sg_batch_commit(sg_ctx* c, void* stream, const sg_table_desc* tables, uint32
                              "roots download");
     for (uint32_t s = 0; s < k; ++s)
         if (streams[s]) cuda_ok(cudaStreamSynchronize(streams[s]), "sync");
-    cuda_ok(cudaStreamSynchronize(caller), "sync");
+    const int rs = sync_checked(ctx, caller, "batch commit");
+    if (rc == SG_OK) rc = rs;
     dev_free(ctx, caller, d_roots, 32ull * count);
     for (uint32_t s = 0; s < k; ++s) {
         if (done[s]) cudaEventDestroy(done[s]);
@@ -940,11 +951,11 @@ int sg_batch_commit_fused(sg_ctx* c, void* stream, const sg_table_desc* tables, 
     std::vector<uint8_t> roots(32ull * count);
     if (rc == SG_OK) {
         cudaError_t e = cudaMemcpyAsync(roots.data(), d_roots, 32ull * count, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
             set_error(std::string("fused batch commit: ") + cudaGetErrorString(e));
             rc = SG_ERR_CUDA;
         }
+        if (rc == SG_OK) rc = sync_checked(ctx, st, "fused batch commit");
     }
     for (uint32_t s = 0; s < k; ++s) {
         if (streams[s]) {

@@ -115,10 +115,15 @@ struct Ctx {
     // Learned pass-cost model (mlp.cu): when set, DFT tile widths are its choice.
     std::vector<float> pass_model;
     // One page-locked word that a kernel sets when a bounded wait of its ran
-    // out (ntt_tc.cu); null in contexts that do not allocate. The launch check
-    // and sg_stream_sync report it.
+    // out (ntt_tc.cu, rounds.cu k_bary_tc); null in contexts that do not
+    // allocate. Every launch check and every wait that makes results visible
+    // to the host reports it, from then on: which results are spoiled is not
+    // known, so the word is never cleared.
     volatile unsigned* fault_host = nullptr;
     unsigned* fault_dev = nullptr;
+    // Failure injection for tests: when > 0, the launch that brings the count
+    // to zero sets the word behind its own check.
+    std::atomic<int64_t> fail_wait_after{-1};
 };
 
 // Host-side prediction of the pass-cost model (mlp.cu): log(ms) for features x.
@@ -210,6 +215,22 @@ inline int check_launch(Ctx* ctx, const char* what) {
         return SG_ERR_CUDA;
     }
     ctx->launches.fetch_add(1, std::memory_order_relaxed);
+    const int rc = check_fault(ctx);
+    if (ctx->fail_wait_after.load(std::memory_order_relaxed) > 0 && ctx->fail_wait_after.fetch_sub(1) == 1 &&
+        ctx->fault_host)
+        *ctx->fault_host = 1;
+    return rc;
+}
+
+// Wait for the stream before results of its kernels are handed to the host. A
+// launch is checked when it is enqueued, before its waits have been tried, so
+// the error word is looked at here again.
+inline int sync_checked(Ctx* ctx, cudaStream_t st, const char* what) {
+    cudaError_t e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        set_error(std::string(what) + ": " + cudaGetErrorString(e));
+        return SG_ERR_CUDA;
+    }
     return check_fault(ctx);
 }
 

@@ -792,10 +792,7 @@ int sg_eval_constraints(sg_ctx* c, void* stream, const sg_device_program* prog, 
                                                              use_smem ? nullptr : d_scr, d_extra);
             rc = check_launch(ctx, "k_constraints");
         }
-        if (rc == SG_OK && cudaStreamSynchronize(st) != cudaSuccess) {
-            set_error("constraints: execution failed");
-            rc = SG_ERR_CUDA;
-        }
+        if (rc == SG_OK) rc = sync_checked(ctx, st, "constraints");
         if (d_cm) dev_free(ctx, st, d_cm, cm_bytes);
         if (d_extra) dev_free(ctx, st, d_extra, extra_bytes);
     }

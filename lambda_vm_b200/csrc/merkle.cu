@@ -425,12 +425,13 @@ extern "C" int sg_grind(sg_ctx* c, void* stream, const uint64_t inner_lanes[4], 
             if (rc != SG_OK) break;
             e = cudaMemcpyAsync(&host, d_best, 8, cudaMemcpyDeviceToHost, st);
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
             set_error(std::string("grind: ") + cudaGetErrorString(e));
             rc = SG_ERR_CUDA;
             break;
         }
+        rc = sync_checked(ctx, st, "grind");
+        if (rc != SG_OK) break;
         if (host != ~0ULL) {
             *nonce_out = host;
             break;

@@ -249,11 +249,11 @@ int sg_mlp_train(sg_ctx* c, void* stream, const float* d_x, const float* d_y, ui
     if (rc == SG_OK) rc = loss_grad(ctx, st, d_x, d_y, n, d_params, grad, loss, partial, lp);
     if (rc == SG_OK && loss_out) {
         cudaError_t e = cudaMemcpyAsync(loss_out, loss, 4, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
             set_error(std::string("mlp train: ") + cudaGetErrorString(e));
             rc = SG_ERR_CUDA;
         }
+        if (rc == SG_OK) rc = sync_checked(ctx, st, "mlp train");
     }
     dev_free(ctx, st, mem, words * 4);
     return rc;

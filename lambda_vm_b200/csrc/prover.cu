@@ -105,7 +105,7 @@ int commit_rows(Ctx* ctx, cudaStream_t st, Bufs& b, const uint64_t* d_rows, uint
     SG_TRY(leaves_row_major(ctx, st, d_rows, rows, row_u64, 0, row_u64, 2, 0, nodes + (L - 1) * 32));
     SG_TRY(merkle_inner(ctx, st, nodes, L));
     SG_CUDA(cudaMemcpyAsync(root, nodes, 32, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
+    SG_TRY(sync_checked(ctx, st, "prove table"));
     *nodes_out = nodes;
     return SG_OK;
 }
@@ -257,7 +257,7 @@ extern "C" int sg_prove_table(sg_ctx* c, void* stream, sg_transcript* t, const s
                                d_S + 6 * m + 6 * A));
     std::vector<uint64_t> S((2 * m + 2 * A + 2) * 3);
     SG_CUDA(cudaMemcpyAsync(S.data(), d_S, S.size() * 8, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
+    SG_TRY(sync_checked(ctx, st, "prove table"));
     bf.release(d_invd);
     bf.release(d_S);
     // round 4's denominators depend on z only: they are inverted while the
@@ -375,7 +375,7 @@ extern "C" int sg_prove_table(sg_ctx* c, void* stream, sg_transcript* t, const s
         SG_TRY(fri_fold_dev(ctx, st, ev, h, tw, d_zeta, evf, twf, nullptr));
         std::vector<uint8_t> back(state_bytes + roots_bytes + h * 24);
         SG_CUDA(cudaMemcpyAsync(back.data(), d_back, back.size(), cudaMemcpyDeviceToHost, st));
-        SG_CUDA(cudaStreamSynchronize(st));
+        SG_TRY(sync_checked(ctx, st, "prove table"));
         memcpy(&t->s, back.data(), sizeof(fs::State));
         memcpy(o->fri_roots, back.data() + state_bytes, roots_bytes);
         final_cw.resize(h * 3);
@@ -384,7 +384,7 @@ extern "C" int sg_prove_table(sg_ctx* c, void* stream, sg_transcript* t, const s
     } else {
         final_cw.resize(ev_len * 3);
         SG_CUDA(cudaMemcpyAsync(final_cw.data(), ev, ev_len * 24, cudaMemcpyDeviceToHost, st));
-        SG_CUDA(cudaStreamSynchronize(st));
+        SG_TRY(sync_checked(ctx, st, "prove table"));
     }
     if (own_tw) bf.release(own_tw);
     const uint64_t term_off = sg_host_gl_pow(g, 1ULL << shp.total_folds);
@@ -471,6 +471,6 @@ extern "C" int sg_prove_table(sg_ctx* c, void* stream, sg_transcript* t, const s
         fri_path_host += Q * (uint64_t)log2_exact(layers[l].leaves) * 32;
     }
     for (auto& x : outs) SG_CUDA(cudaMemcpyAsync(x.host, x.dev, x.bytes, cudaMemcpyDeviceToHost, st));
-    SG_CUDA(cudaStreamSynchronize(st));
+    SG_TRY(sync_checked(ctx, st, "prove table"));
     return SG_OK;  // Bufs releases every device buffer on the stream
 }

@@ -119,11 +119,11 @@ static int with_zero_flag(Ctx* ctx, cudaStream_t st, int* zero_out, F&& launch) 
     if (rc == SG_OK) rc = launch(d_flag);
     if (rc == SG_OK && zero_out) {
         unsigned h = 0;
-        if (cudaMemcpyAsync(&h, d_flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess) {
+        if (cudaMemcpyAsync(&h, d_flag, sizeof(unsigned), cudaMemcpyDeviceToHost, st) != cudaSuccess) {
             set_error("batch inverse: flag readback failed");
             rc = SG_ERR_CUDA;
         }
+        if (rc == SG_OK) rc = sync_checked(ctx, st, "batch inverse");
         *zero_out = h ? 1 : 0;
     }
     int rf = dev_free(ctx, st, d_flag, sizeof(unsigned));
@@ -1073,10 +1073,7 @@ int sg_deep_composition(sg_ctx* c, void* stream, const uint64_t* d_main, uint64_
                                                                         bitrev_out, d_out);
         rc = check_launch(ctx, "k_deep");
         // keep host vectors alive until the copies have been consumed
-        if (rc == SG_OK && cudaStreamSynchronize(st) != cudaSuccess) {
-            set_error("deep: sync failed");
-            rc = SG_ERR_CUDA;
-        }
+        if (rc == SG_OK) rc = sync_checked(ctx, st, "deep");
     }
     int rf = dev_free(ctx, st, d_g, gbytes);
     return rc != SG_OK ? rc : rf;
@@ -1208,11 +1205,11 @@ int sg_logup_aux(sg_ctx* c, void* stream, const uint64_t* d_main, uint64_t n, ui
             k_logup_acc<<<(unsigned)nseg, LG_SEG, 0, st>>>(d_rs, n, d_seg + 6, d_seg, W, d_aux);
             rc = check_launch(ctx, "k_logup_acc");
         }
-        if (rc == SG_OK && (cudaMemcpyAsync(table_contribution, d_seg, 24, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                            cudaStreamSynchronize(st) != cudaSuccess)) {
+        if (rc == SG_OK && cudaMemcpyAsync(table_contribution, d_seg, 24, cudaMemcpyDeviceToHost, st) != cudaSuccess) {
             set_error("logup: contribution readback failed");
             rc = SG_ERR_CUDA;
         }
+        if (rc == SG_OK) rc = sync_checked(ctx, st, "logup");
     }
     dev_free(ctx, st, d_seg, sb);
     dev_free(ctx, st, d_rs, rb);
@@ -1306,11 +1303,11 @@ static int fri_fold_step(sg_fri* f, const uint64_t zeta[3], bool commit, uint8_t
     if (rc == SG_OK && commit && root_out) e = cudaMemcpyAsync(root_out, nodes, 32, cudaMemcpyDeviceToHost, f->st);
     if (rc == SG_OK && e == cudaSuccess && host_evals_out)
         e = cudaMemcpyAsync(host_evals_out, out, 24 * h, cudaMemcpyDeviceToHost, f->st);
-    if (rc == SG_OK && e == cudaSuccess) e = cudaStreamSynchronize(f->st);
     if (rc == SG_OK && e != cudaSuccess) {
         set_error(std::string("fri fold: ") + cudaGetErrorString(e));
         rc = SG_ERR_CUDA;
     }
+    if (rc == SG_OK) rc = sync_checked(ctx, f->st, "fri fold");
     if (rc != SG_OK) {
         dev_free(ctx, f->st, out, 24 * h);
         dev_free(ctx, f->st, twn, 8 * (nl ? nl : 1));

@@ -226,11 +226,11 @@ extern "C" int sg_verify_queries(sg_ctx* c, void* stream, const sg_verify_table*
         rc = check_launch(ctx, "k_verify_queries");
     }
     if (rc == SG_OK && e == cudaSuccess) e = cudaMemcpyAsync(status_out, ds, total * 4, cudaMemcpyDeviceToHost, st);
-    if (rc == SG_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (rc == SG_OK && e != cudaSuccess) {
         set_error(std::string("verify queries: ") + cudaGetErrorString(e));
         rc = SG_ERR_CUDA;
     }
+    if (rc == SG_OK) rc = sync_checked(ctx, st, "verify queries");
     dev_free(ctx, st, ds, total * 4);
     dev_free(ctx, st, dd, count * sizeof(VerifyDesc));
     return rc;

@@ -38,6 +38,9 @@ class Backend:
     def fail_alloc_after(self, n: int):
         native.check(native.lib().sg_ctx_fail_alloc_after(self.h, n))
 
+    def fail_wait_after(self, n: int):
+        native.check(native.lib().sg_ctx_fail_wait_after(self.h, n))
+
     def sync(self, stream=None):
         native.check(native.lib().sg_stream_sync(self.h, stream))
 

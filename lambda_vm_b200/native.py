@@ -112,6 +112,7 @@ PROTOTYPES = {
     "sg_ctx_launches": (u64, [vp]),
     "sg_ctx_budget": (u64, [vp]),
     "sg_ctx_fail_alloc_after": (i32, [vp, C.c_int64]),
+    "sg_ctx_fail_wait_after": (i32, [vp, C.c_int64]),
     "sg_dev_alloc": (i32, [vp, vp, u64, C.POINTER(vp)]),
     "sg_dev_free": (i32, [vp, vp, vp, u64]),
     "sg_memcpy_h2d": (i32, [vp, vp, vp, vp, u64]),

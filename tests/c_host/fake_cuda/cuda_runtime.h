@@ -16,4 +16,5 @@ typedef void* cudaEvent_t;
 cudaError_t cudaGetDevice(int* device);
 cudaError_t cudaSetDevice(int device);
 cudaError_t cudaGetLastError(void);
+cudaError_t cudaStreamSynchronize(cudaStream_t stream);
 const char* cudaGetErrorString(cudaError_t e);
