@@ -11,6 +11,7 @@
 //  * LogUp:       lookup.rs:1660-1842 with the CSR descriptor of
 //                 crypto/math-cuda/src/logup.rs:26-44.
 // All layouts are row-major; ext3 values are 3 consecutive u64.
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -237,6 +238,18 @@ __global__ void __launch_bounds__(256) k_inv_denoms(const uint64_t* __restrict__
 // still fill the block and each warp reads whole row segments. The lanes'
 // sums meet in the same shared memory; one partial per (chunk, k, column)
 // goes to k_bary_combine.
+//
+// A thread holds 3 K sums. In the eight-word form they fit beside the loop's
+// operands up to K = 3 (ext3) and K = 4 (base; at K = 2 they cost a block an
+// SM); beyond, in 128 registers, the compiler spills every one of them: 2^19
+// rows x 80 base columns, K = 5: 7870 us against 688 with the five-limb form,
+// x 20 ext3 columns 4481 against 483. Eight words against five below that, the
+// same rows: base K = 2 (x 3) 58 against 45, K = 3 409 against 459, K = 4 520
+// against 575; ext3 K = 1, 2, 3 116, 206, 263 against 135, 236, 326, K = 4 409
+// against 402.
+template <bool EXT3, int K>
+using bary_acc =
+    std::conditional_t<EXT3 ? K <= 3 : (K == 1 || K == 3 || K == 4), gl::wacc3, gl::nacc3>;
 template <bool EXT3, int K>
 __global__ void __launch_bounds__(512) k_bary(const uint64_t* __restrict__ data, uint64_t row_u64, uint64_t stride,
                                               uint64_t cols, uint32_t CT, uint32_t RL, uint32_t RB,
@@ -247,11 +260,11 @@ __global__ void __launch_bounds__(512) k_bary(const uint64_t* __restrict__ data,
     const uint32_t lane = threadIdx.x / CT, cl = threadIdx.x % CT;
     const uint64_t c = (uint64_t)blockIdx.x * CT + cl;
     const bool active = lane < RL && c < cols;
-    // Row sums are accumulated unreduced (160-bit, at most 3n products each)
-    // and reduced once per thread.
-    gl::wacc3 wa[K];
+    // Row sums are accumulated unreduced (at most 3n products each) and
+    // reduced once per thread.
+    bary_acc<EXT3, K> wa[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) wa[k] = gl::wzero3();
+    for (int k = 0; k < K; ++k) wa[k] = {};
     const uint64_t i0 = blockIdx.y * chunk_len, i1 = min(n, i0 + chunk_len);
     for (uint64_t b0 = i0; b0 < i1; b0 += RB) {
         const uint32_t nb = (uint32_t)min((uint64_t)RB, i1 - b0);

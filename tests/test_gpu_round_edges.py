@@ -123,3 +123,43 @@ def test_table_kernels_at_tile_edges(be, table, rows, step):
     for comp in comps:
         want = mc.eval_constraints_on_device(full, main, aux, *rest, comp, be)
         assert np.array_equal(mc.eval_constraints_on_device(dev, main, aux, *rest, comp, be), want)
+
+
+# The general kernel holds its 3 k sums in eight words or in five limbs each,
+# by ext3 and k: largest words, and rows that end inside a batch.
+@pytest.mark.parametrize("ext3", [False, True])
+@pytest.mark.parametrize("k", range(1, 9))
+def test_barycentric_sums_of_every_point_count(be, ext3, k):
+    n, cols = 1037, 5
+    data = np.full((n, 17), 2**64 - 1, np.uint64)
+    pts, invd = np.full(n, P - 1, np.uint64), np.full(3 * k * n, P - 1, np.uint64)
+    invd[::7] = np.random.default_rng(k).integers(0, P, invd[::7].size, dtype=np.uint64)
+    got = mc.barycentric_multi(data, 1, ext3, cols, pts, invd, n, k, be)
+    assert (got == O.canon_array(O.barycentric_sums(data, 1, ext3, cols, pts, invd, n, k))).all()
+
+
+@pytest.mark.parametrize("ext3", [False, True])
+def test_barycentric_time_grows_with_the_point_count(be, ext3):
+    """Sums that do not fit the registers cost ten times their arithmetic: 5 to
+    8 points take about 1.3 to 2.7 times as long as 4, never more than 5."""
+    import torch
+    from lambda_vm_b200 import native
+    n, cols, w = 1 << 17, 20, 3 if ext3 else 1
+    data = torch.ones(n * cols * w, dtype=torch.int64, device="cuda")
+    pts, invd = (torch.ones(q, dtype=torch.int64, device="cuda") for q in (n, 24 * n))
+    out = torch.empty(3 * 8 * cols, dtype=torch.int64, device="cuda")
+
+    def ms(k):
+        best = []
+        for _ in range(6):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            native.check(native.lib().sg_barycentric_sums(be.h, None, data.data_ptr(), cols * w, 1, int(ext3), cols,
+                                                          pts.data_ptr(), invd.data_ptr(), n, k, out.data_ptr()))
+            e1.record()
+            e1.synchronize()
+            best.append(e0.elapsed_time(e1))
+        return min(best)
+
+    base = ms(4)
+    assert all(ms(k) < 5 * base for k in range(5, 9))
