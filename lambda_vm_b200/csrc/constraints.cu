@@ -753,8 +753,9 @@ int sg_eval_constraints(sg_ctx* c, void* stream, const sg_device_program* prog, 
             const uint64_t hb = (rows + 127) / 128, hcap = 148ull * 16;
             const unsigned grid = (unsigned)(hb < hcap ? hb : hcap);
             if (hand_id == SG_AIR_KECCAK) {
-                k_keccak_constraints<<<grid, 128, 0, st>>>(d_cm, d_main, rows, next_step, keccak_consts(),
-                                                           d_blob + o_beta, comp ? 0 : 1, comp ? d_extra : d_out);
+                auto kernel = hb <= 5ull * sms ? k_keccak_constraints<5> : k_keccak_constraints<7>;
+                kernel<<<grid, 128, 0, st>>>(d_cm, d_main, rows, next_step, keccak_consts(), d_blob + o_beta,
+                                             comp ? 0 : 1, comp ? d_extra : d_out);
                 rc = check_launch(ctx, "k_keccak_constraints");
             } else if (hand_id == SG_AIR_SHIFT) {
                 k_shift_constraints<<<grid, 128, 0, st>>>(d_cm, d_main, rows, next_step, d_blob + o_beta,

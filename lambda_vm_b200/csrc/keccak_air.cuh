@@ -143,7 +143,15 @@ __device__ __forceinline__ uint64_t kchi(const KRow& w, const KeccakConsts& kc, 
 //   3069 + 4 (5 X + Y - 1) + l: OUT limb l of lane (X, Y) != (0, 0) from chi;
 //   3165 + z: lane 0's chi bit; 3229 + l: lane 0's OUT limb after iota;
 //   3233.. the transitions and the timestamp gaps, in program order.
-static __global__ void k_keccak_constraints(const uint64_t* __restrict__ cm, const uint64_t* __restrict__ rm, uint64_t rows,
+//
+// Bound by the latency of its column loads, so by warps in flight: one CTA
+// more or less a wave decides. CTAS is the CTAs an SM holds: 5 (96 registers,
+// loads issued furthest ahead) while that is one wave, else 7 (72 registers).
+// A composition of 2^16 rows (512 CTAs): 4.20 ms with 5, 4.39 with 7; 2^17
+// (1024 CTAs, two waves of 740 or one of 1036): 7.38 and 6.95; 2^18: 12.71
+// and 12.66.
+template <int CTAS>
+static __global__ void __launch_bounds__(128, CTAS) k_keccak_constraints(const uint64_t* __restrict__ cm, const uint64_t* __restrict__ rm, uint64_t rows,
                                      uint64_t next_step, KeccakConsts kc, const uint64_t* __restrict__ beta, int mode,
                                      uint64_t* __restrict__ out) {
     for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < rows;

@@ -163,3 +163,19 @@ def test_barycentric_time_grows_with_the_point_count(be, ext3):
 
     base = ms(4)
     assert all(ms(k) < 5 * base for k in range(5, 9))
+
+
+def test_keccak_table_beyond_one_wave(be):
+    """From 741 blocks of rows on the KECCAK constraints run in the form that
+    holds seven blocks an SM: rows that repeat a short table's give its values."""
+    import torch
+    air = RA.KeccakAir(8)
+    dev = lower(air.device_program)
+    rng = np.random.default_rng(4)
+    main, aux = rf(rng, (128, air.width)), rf(rng, (128, 3 * air.aux_width))
+    comp = {"beta": rf(rng, (dev["num_roots"], 3)), "z_inv": rf(rng, (4,))}
+    rest = rf(rng, (2, 3)), rf(rng, (air.max_alpha, 3)), rf(rng, (3,)), 2, comp, be
+    reps = 5 * torch.cuda.get_device_properties(0).multi_processor_count + 1
+    want = mc.eval_constraints_on_device(dev, main, aux, *rest)
+    got = mc.eval_constraints_on_device(dev, np.tile(main, (reps, 1)), np.tile(aux, (reps, 1)), *rest)
+    assert np.array_equal(got, np.tile(want, (reps, 1)))
