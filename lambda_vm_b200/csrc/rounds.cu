@@ -62,17 +62,50 @@ __device__ __forceinline__ bool is_zero3(fe3 v) {
 // one thread's chain).
 #define BI_CH 12
 
-__global__ void __launch_bounds__(256) k_batch_inv(const uint64_t* in, uint64_t total, uint64_t* out,
-                                                   unsigned* zero_flag) {
+struct LoadPlain {
+    const uint64_t* in;
+    struct Cur {
+        uint64_t base;
+    };
+    __device__ __forceinline__ Cur start(uint64_t base) const { return Cur{base}; }
+    __device__ __forceinline__ fe3 at(const Cur& c, int j) const { return ld3(in + 3 * (c.base + j)); }
+};
+// Denominators z_k - x_i (x_minus_z 0) or x_i - z_k (1), element k n + i, of
+// calls with few points and many z (sg_inv_denoms_ext3). A thread's cursor
+// divides once; its later elements step (k, i) forward.
+struct LoadDenom {
+    const uint64_t* x;
+    const uint64_t* z;
+    uint64_t n;
+    int x_minus_z;
+    struct Cur {
+        uint64_t k, i;
+    };
+    __device__ __forceinline__ Cur start(uint64_t base) const {
+        const uint64_t k = base / n;
+        return Cur{k, base - k * n};
+    }
+    __device__ __forceinline__ fe3 at(const Cur& c, int j) const {
+        uint64_t k = c.k, i = c.i + (uint64_t)j;
+        while (i >= n) i -= n, ++k;
+        const fe3 zk = ld3(z + 3 * k);
+        const uint64_t xi = x[i];
+        return x_minus_z ? fe3{gl::sub(xi, zk.c0), gl::neg(zk.c1), gl::neg(zk.c2)}
+                         : fe3{gl::sub(zk.c0, xi), zk.c1, zk.c2};
+    }
+};
+
+template <class Load>
+__global__ void __launch_bounds__(256) k_batch_inv(Load load, uint64_t total, uint64_t* out, unsigned* zero_flag) {
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t base = tid * BI_CH;
     const int lane = threadIdx.x & 31;
-    auto at = [&](int j) { return ld3(in + 3 * (base + j)); };
+    const typename Load::Cur cur = load.start(base < total ? base : 0);
     // prefix products of the chunk; elements past the end count as 1
     fe3 p[BI_CH];
-    p[0] = base < total ? at(0) : one3();
+    p[0] = base < total ? load.at(cur, 0) : one3();
 #pragma unroll
-    for (int i = 1; i < BI_CH; ++i) p[i] = base + i < total ? gl::mul3(p[i - 1], at(i)) : p[i - 1];
+    for (int i = 1; i < BI_CH; ++i) p[i] = base + i < total ? gl::mul3(p[i - 1], load.at(cur, i)) : p[i - 1];
     const fe3 tot = p[BI_CH - 1];
     fe3 incl = tot, sinc = tot;
 #pragma unroll
@@ -98,7 +131,7 @@ __global__ void __launch_bounds__(256) k_batch_inv(const uint64_t* in, uint64_t 
 #pragma unroll
     for (int i = BI_CH - 1; i >= 1; --i) {
         if (base + i < total) {
-            const fe3 a = at(i);  // before the store: out may alias the input
+            const fe3 a = load.at(cur, i);  // before the store: out may alias the input
             st3(out + 3 * (base + i), gl::canon3(gl::mul3(inv, p[i - 1])));
             inv = gl::mul3(inv, a);
         }
@@ -131,12 +164,12 @@ static int with_zero_flag(Ctx* ctx, cudaStream_t st, int* zero_out, F&& launch) 
     return rc != SG_OK ? rc : rf;
 }
 
-static int batch_inv_launch(Ctx* ctx, cudaStream_t st, const uint64_t* in, uint64_t total, uint64_t* out,
-                            int* zero_out) {
+template <class Load>
+static int batch_inv_launch(Ctx* ctx, cudaStream_t st, Load load, uint64_t total, uint64_t* out, int* zero_out) {
     if (total == 0) return SG_OK;
     return with_zero_flag(ctx, st, zero_out, [&](unsigned* d_flag) {
         const uint64_t threads = (total + BI_CH - 1) / BI_CH;
-        k_batch_inv<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(in, total, out, d_flag);
+        k_batch_inv<Load><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(load, total, out, d_flag);
         return check_launch(ctx, "k_batch_inv");
     });
 }
@@ -152,8 +185,8 @@ static int batch_inv_launch(Ctx* ctx, cudaStream_t st, const uint64_t* in, uint6
 // thread `lane` the points lane, lane + 32, ...: points are read and results
 // written (through shared memory) in whole segments; a warp prefix and suffix
 // scan of the threads' products leaves one base-field inversion a warp.
-// CH: 16 where that fills the schedulers, 4 below (a thread's chain is the
-// latency there).
+// CH: 16 where that fills the schedulers (sg_inv_denoms_ext3), 4 below (a
+// thread's chain is the latency there).
 template <int CH>
 __global__ void __launch_bounds__(256) k_inv_denoms(const uint64_t* __restrict__ x, const uint64_t* __restrict__ z,
                                                     uint64_t n, int x_minus_z, uint64_t* __restrict__ out,
@@ -910,7 +943,7 @@ int sg_batch_inverse_ext3(sg_ctx* c, void* stream, const uint64_t* d_in, uint64_
                           int* zero_found) {
     SG_CHECK_ARG(c && (n == 0 || (d_in && d_out)), "null argument");
     SG_ENTER(ctx_of(c));
-    return batch_inv_launch(CX(c), (cudaStream_t)stream, d_in, n, d_out, zero_found);
+    return batch_inv_launch(CX(c), (cudaStream_t)stream, LoadPlain{d_in}, n, d_out, zero_found);
 }
 
 int sg_inv_denoms_ext3(sg_ctx* c, void* stream, const uint64_t* d_x, uint64_t n, const uint64_t* z_host, uint32_t k,
@@ -927,10 +960,19 @@ int sg_inv_denoms_ext3(sg_ctx* c, void* stream, const uint64_t* d_x, uint64_t n,
         set_error("inv_denoms: z upload failed");
         rc = SG_ERR_CUDA;
     }
-    if (rc == SG_OK)
+    // A CTA of the norms' kernel takes points of one z only: with few points
+    // and many z its warps idle and every z costs an inversion, so those are
+    // inverted as one flat batch (96 points x 16384 z: 103 us flat, 115 by
+    // norms; x 4096 z: 48 and 41; 128 points x 16384: 130 and 121).
+    if (rc == SG_OK && n < 128 && k > 4096)
+        rc = batch_inv_launch(ctx, st, LoadDenom{d_x, d_z, n, x_minus_z}, n * k, d_out, zero_found);
+    else if (rc == SG_OK)
         rc = with_zero_flag(ctx, st, zero_found, [&](unsigned* d_flag) {
-            // 16 points a thread once that gives every scheduler a few warps
-            const bool wide = n * k >= (1ULL << 20);
+            // 16 points a thread, where that still gives every scheduler a
+            // warp and a CTA's warps enough points (2^18 points x 2 z: 25 us,
+            // with 4 a thread 29; 2^17 x 3: 26 and 24; 2000 x 1024: 72 and
+            // 82; 1024 x 1024: 78 and 46)
+            const bool wide = n >= 1792 && n * k >= (1ULL << 19);
             const uint64_t per = 256ull * (wide ? 16 : 4);
             for (uint32_t k0 = 0; k0 < k; k0 += 65535) {  // grid.y limit
                 const dim3 grid((unsigned)((n + per - 1) / per), k - k0 < 65535 ? k - k0 : 65535);
@@ -1195,7 +1237,7 @@ int sg_logup_aux(sg_ctx* c, void* stream, const uint64_t* d_main, uint64_t n, ui
             k_logup_fp<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(d_main, n, m, d, z[0], z[1], z[2], d_fp);
             rc = check_launch(ctx, "k_logup_fp");
             int zf = 0;
-            if (rc == SG_OK) rc = batch_inv_launch(ctx, st, d_fp, tot, d_fp, &zf);
+            if (rc == SG_OK) rc = batch_inv_launch(ctx, st, LoadPlain{d_fp}, tot, d_fp, &zf);
             if (rc == SG_OK && zf) {
                 set_error("logup: a fingerprint is zero (challenge collides with a row value)");
                 rc = SG_ERR_INVALID;

@@ -19,9 +19,12 @@ def rf(rng, shape):
     return np.where(x >= np.uint64(P), x - np.uint64(P), x)
 
 
-# 2^20 denominators and more run 16 a thread (512 a warp), fewer 4 (128 a warp)
+# From 1792 points and 2^19 denominators on 16 a thread (512 a warp), else 4
+# (128 a warp); fewer than 128 points of more than 4096 z as one flat batch
 @pytest.mark.parametrize("n,k,sign", [(127, 2, 0), (129, 3, 1), (1024, 1, 0), (1 << 20, 1, 1), ((1 << 19) + 1, 2, 0),
-                                      ((1 << 20) - 511, 2, 1), (300007, 5, 0)])
+                                      ((1 << 20) - 511, 2, 1), (300007, 5, 0),
+                                      (1 << 18, 2, 0), ((1 << 18) - 1, 2, 1), (1792, 300, 1), (1791, 300, 0),
+                                      (1, 4097, 0), (127, 4097, 1), (127, 4096, 0), (128, 4097, 1), (5, 70000, 0)])
 def test_denominators(be, n, k, sign):
     rng = np.random.default_rng(n + k)
     x, z = rf(rng, (n,)), rf(rng, (k, 3))
@@ -34,6 +37,33 @@ def test_zero_denominator_is_reported(be):
     x = np.arange(1, 5001, dtype=np.uint64)
     with pytest.raises(ZeroDivisionError):
         mc.compute_and_invert_denoms_ext3(x, np.array([[7, 1, 2], [4321, 0, 0]], np.uint64), 1, be)
+    z = np.tile(np.array([7, 1, 2], np.uint64), (4100, 1))
+    z[4097] = 9, 0, 0
+    with pytest.raises(ZeroDivisionError):
+        mc.compute_and_invert_denoms_ext3(x[:20], z, 0, be)
+
+
+def test_many_points_z_cost_no_more_than_their_number(be):
+    """8 points of 2^18 z are as many denominators as 2^21 points of one z and
+    take about four times as long as one flat batch, not a hundred times."""
+    import torch
+    from lambda_vm_b200 import native
+    x = torch.arange(1, (1 << 21) + 1, dtype=torch.int64, device="cuda")
+    out = torch.empty(3 << 21, dtype=torch.int64, device="cuda")
+
+    def ms(n, k):
+        z, best = np.arange(3 * k, dtype=np.uint64) + np.uint64(5), []
+        for _ in range(4):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            native.check(native.lib().sg_inv_denoms_ext3(be.h, None, x.data_ptr(), n, z.ctypes.data, k, 1,
+                                                         out.data_ptr(), None))
+            e1.record()
+            e1.synchronize()
+            best.append(e0.elapsed_time(e1))
+        return min(best)
+
+    assert ms(8, 1 << 18) < 20 * ms(1 << 21, 1)
 
 
 # From 2^15 rows and 12 base columns on, one or two points: column tiles of at
