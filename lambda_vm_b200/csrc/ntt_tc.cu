@@ -530,17 +530,47 @@ int launch_kind(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntiles) {
                               : launch<LR1, LR2, DBL, true, FLAT, 3>(ctx, st, a, ntiles);
 }
 
+// Columns of a tile of 2^logL points (TcPlan::CSL).
+uint64_t tile_cols(uint32_t logL) { return PTS >> logL; }
+
+// Columns in tiles of their own leave the last one partly empty; narrow
+// matrices (LogUp columns, composition parts) take their slots from the flat
+// list of (tile, column) pairs instead, at one product more a point: worth it
+// from an eighth of the slots (2^18 x 77, blowup 2, a fifth empty: 1.10 ms
+// against 1.03 flat).
+bool flat_tiles(uint64_t m, uint64_t csl) { return (m + csl - 1) / csl * csl * 8 > m * 9; }
+
+// Whether a short pass is quicker here than on the integer pipes. All SMs take
+// a tile each and the last round is as long as a full one, while k_dft's time
+// grows with its points, columns padded to its narrowest tile; so a pass of
+// 70 or of 150 tiles may be the slower one here. Both times in tenths of a
+// microsecond, fitted to 944 passes of LDEs of 2^7..2^22 rows x 1..600
+// columns, blowup 1 to 16: the quicker kernel is taken but for eight passes
+// that lose 3 to 20 %. 2^14 x 77, blowup 2: 116 us with every pass over 2^20
+// points here, 91 without any. Passes of 2^10 and 2^11 points are quicker here
+// at every size measured (1.14 to 5 times), and so are those over more than
+// two cosets, which k_dft runs one after another in a tile (up to 5 times).
+bool quicker_here(const PassArgs& a, uint64_t ntiles) {
+    if (a.logL > 9 || a.reps > 2) return true;
+    struct Times {
+        uint64_t round, lead, mpoint;  // a round here; what k_dft starts later, its time for 2^20 points
+    };
+    static constexpr Times T[3] = {{140, 10, 85}, {146, 50, 91}, {164, 30, 107}};  // 2^7, 2^8, 2^9 points
+    const Times& t = T[a.logL - 7];
+    const uint64_t csl = tile_cols(a.logL), narrowest = a.logL == 7 ? 32 : 4, ctas = 148 / a.reps;
+    const bool flat = flat_tiles(a.m, csl);
+    const uint64_t tiles = flat ? (ntiles * a.m + csl - 1) / csl : ntiles * ((a.m + csl - 1) / csl);
+    const uint64_t rounds = (tiles + ctas - 1) / ctas;
+    const uint64_t padded = ((a.m + narrowest - 1) / narrowest * narrowest * ntiles * a.reps) << a.logL;
+    const uint64_t more = (flat ? 8 : 0) + (a.inverse ? 15 : a.post_kind == 1 ? 10 : 0);
+    return rounds * (t.round + more) <= t.lead + (t.mpoint * padded >> 20);
+}
+
 template <int LR1, int LR2, bool DBL>
 int launch_len(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntiles) {
-    // Columns in tiles of CSL leave the last one partly empty; narrow matrices
-    // (LogUp columns, composition parts) take their slots from the flat list
-    // of (tile, column) pairs instead, at one product more a point: worth it
-    // from an eighth of the slots (2^18 x 77, blowup 2, a fifth empty: 1.10 ms
-    // against 1.03 flat).
-    constexpr uint64_t CSL = TcPlan<LR1, LR2, DBL, false>::CSL;
-    const bool flat = (a.m + CSL - 1) / CSL * CSL * 8 > a.m * 9;
-    return flat ? launch_kind<LR1, LR2, DBL, true>(ctx, st, a, ntiles)
-                : launch_kind<LR1, LR2, DBL, false>(ctx, st, a, ntiles);
+    static_assert(TcPlan<LR1, LR2, DBL, false>::CSL == PTS >> (LR1 + LR2 + DBL), "columns of a tile");
+    return flat_tiles(a.m, tile_cols(a.logL)) ? launch_kind<LR1, LR2, DBL, true>(ctx, st, a, ntiles)
+                                              : launch_kind<LR1, LR2, DBL, false>(ctx, st, a, ntiles);
 }
 
 }  // namespace
@@ -559,10 +589,8 @@ bool dft_tc_takes(const PassArgs& a, uint64_t ntiles) {
     // 32-bit tile and column arithmetic
     if (a.m >= (1ull << 24) || ntiles * a.m >= (1ull << 31)) return false;
     // Set-up (matrices, twiddles, TMEM) costs a CTA about 8 us and a tile takes
-    // another 8: below about 64 tiles the integer kernel's many small CTAs are
-    // quicker (2^16 x 16, blowup 2, passes of 2^20 and 2^21 points, 16-column
-    // tiles: 79 against 86 us; 2^16 x 33: 187 against 124 us).
-    return L * ntiles * a.m * a.reps > TC_MIN_POINTS;
+    // another 8: up to 64 tiles the integer kernel's many small CTAs are quicker.
+    return L * ntiles * a.m * a.reps > TC_MIN_POINTS && quicker_here(a, ntiles);
 }
 
 int launch_dft_tc(Ctx* ctx, cudaStream_t st, const PassArgs& a, uint64_t ntiles) {

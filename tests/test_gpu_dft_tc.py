@@ -67,3 +67,16 @@ def test_extreme_words(be):
         got, tc = tensor_passes(be, lambda: mc.coset_lde_batch_base(t, 2, w, be))
         assert tc
         assert (got == O.canon_array(O.coset_lde_row_major(t, 2, w))).all()
+
+
+# Passes of 2^7 to 2^9 points whose last round of tiles is nearly empty stay on
+# the integer pipes: the shape's whole LDE, some of its passes, or none.
+@pytest.mark.parametrize("log_n,m,blowup,on_tensor_cores", [
+    (14, 77, 2, []), (13, 150, 2, []), (14, 300, 2, [(7, 0, 1), (7, 0, 0)]), (15, 77, 2, [(7, 0, 1), (8, 0, 0)]),
+    (16, 24, 2, [(8, 1, 1), (8, 1, 2), (8, 0, 0)])])
+def test_short_passes_take_the_quicker_kernel(be, log_n, m, blowup, on_tensor_cores):
+    n = 1 << log_n
+    t, w = raw(log_n * 31 + m, (n, m)), O.coset_weights(n, 3)
+    got, tc = tensor_passes(be, lambda: mc.coset_lde_batch_base(t, blowup, w, be))
+    assert tc == on_tensor_cores
+    assert (got == O.canon_array(O.coset_lde_row_major(t, blowup, w))).all()
