@@ -211,9 +211,9 @@ __global__ void __launch_bounds__(NT + 32, 1)
     uint64_t* W = reinterpret_cast<uint64_t*>(sm8 + PL::OFF_W);    // DBL: w_2T^i
     // Barriers: an accumulator's product is complete (per accumulator), the 16
     // warps have read it (per accumulator), the tile's inputs have landed, and
-    // stage 1's outputs are in A.
+    // stage 1's outputs are in A; the last one is for a CTA that gives up.
     const uint32_t bar_full = smem_addr(sm8 + PL::OFF_BAR), bar_read = bar_full + 16, bar_loaded = bar_full + 32,
-                   bar_ready = bar_full + 40;
+                   bar_ready = bar_full + 40, bar_drain = bar_full + 56;
     uint32_t* ctrl = reinterpret_cast<uint32_t*>(sm8 + PL::OFF_BAR + 48);  // TMEM address, abort word
     volatile uint32_t* abort = ctrl + 1;
     const uint64_t mask = (1ull << a.tw.logN) - 1;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(NT + 32, 1)
     if (tid == 0) {
         mbar_init(bar_full, 1), mbar_init(bar_full + 8, 1);
         mbar_init(bar_read, NT / 32), mbar_init(bar_read + 8, NT / 32);
-        mbar_init(bar_loaded, NT), mbar_init(bar_ready, NT / 32);
+        mbar_init(bar_loaded, NT), mbar_init(bar_ready, NT / 32), mbar_init(bar_drain, 1);
         *abort = 0;
     }
     const uint32_t r2 = R1 == R2 ? rep : 0;  // one matrix serves both stages when R1 == R2
@@ -262,7 +262,8 @@ __global__ void __launch_bounds__(NT + 32, 1)
         // ---- the issuing warp: every step's products as soon as their inputs
         // are there and their accumulator has been read
         uint32_t uses = 0;  // of each accumulator so far
-        for (uint32_t t = t0, n = 0; t < gtiles && !*abort; t += gstep, ++n) {
+        auto gave_up = [&] { return __any_sync(0xffffffffu, *abort != 0); };  // one answer for the warp
+        for (uint32_t t = t0, n = 0; t < gtiles && !gave_up(); t += gstep, ++n) {
 #pragma unroll 1
             for (uint32_t st = 0; st < 2; ++st) {
                 mbar_wait(st ? bar_ready : bar_loaded, n & 1, abort, err);
@@ -284,6 +285,11 @@ __global__ void __launch_bounds__(NT + 32, 1)
                     if (b) ++uses;
                 }
             }
+        }
+        if (gave_up()) {
+            if (elect_one()) mma_commit(bar_drain);
+            __syncwarp();
+            mbar_drain(bar_drain, 0);
         }
         __syncthreads();
         tc_after();
@@ -493,8 +499,8 @@ __global__ void __launch_bounds__(NT + 32, 1)
             loaded();
         }
     }
-    // every product has been waited for above, except after a timeout: the
-    // accumulators' columns are then given back all the same
+    // every product has been waited for above; after a timeout the issuing warp
+    // waits for those in flight, and the columns are given back all the same
     copy_async_wait();
     tc_before();
     __syncthreads();

@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2)
             }
         }
         fence_async();
-        __syncthreads();
+        if (__syncthreads_or(*abort != 0)) break;  // a wait ran out: all threads leave
         if (warp == 0) {
             tc_after();
             if (elect_one()) {
@@ -504,10 +504,12 @@ __global__ void __launch_bounds__(BT_THREADS, 2)
         }
     }
     if (turn) mbar_wait(bar, (turn - 1) & 1, abort, err);
+    const bool complete = !__syncthreads_or(*abort != 0);
+    if (!complete && turn) mbar_drain(bar, (turn - 1) & 1);
     tc_after();
     // ---- accumulators: row (b, c), column (q, a); sum_a first, times 2^8b, then over b
     uint64_t* red = reinterpret_cast<uint64_t*>(bt_sm);  // [M-tile][row][q]; the products are done with A
-    for (uint32_t m = warp >> 2; m < mt; m += 2) {
+    for (uint32_t m = warp >> 2; complete && m < mt; m += 2) {
         const uint32_t row = 32 * (warp & 3) + lane;
         const uint64_t scale = 1ull << (8 * (row >> 4));
 #pragma unroll
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2)
     __syncthreads();
     tc_after();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
-    for (uint32_t e = tid; e < ncols * Q; e += BT_THREADS) {
+    for (uint32_t e = tid; complete && e < ncols * Q; e += BT_THREADS) {
         const uint32_t c = e / Q, q = e % Q;
         uint64_t t = 0;
         for (uint32_t b = 0; b < 8; ++b) t = gl::add(t, red[((c >> 4) * 128 + b * 16 + (c & 15)) * Q + q]);

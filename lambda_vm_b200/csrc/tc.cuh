@@ -3,6 +3,8 @@
 #pragma once
 #include <stdint.h>
 
+#include "wait.cuh"
+
 namespace sg {
 namespace tc {
 
@@ -25,20 +27,26 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ uint64_t clock_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// The last wait of a CTA that leaves after a timeout: its products may still
+// read shared memory and write TMEM, so they get two seconds more before both
+// are given back.
+static __device__ __noinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    const uint32_t go_on = 0;
+    bounded_wait([=] { return mbar_try(bar, parity); }, clock_ns, &go_on, WAIT_LIMIT_NS);
+}
 static __device__ __noinline__ void mbar_wait_slow(uint32_t bar, uint32_t parity, volatile uint32_t* abort, unsigned* err) {
-    uint64_t t0, t1;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-    do {
-        for (int i = 0; i < 64; ++i)
-            if (mbar_try(bar, parity)) return;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-    } while (!*abort && t1 - t0 < 2000000000ull);
+    if (bounded_wait([=] { return mbar_try(bar, parity); }, clock_ns, abort, WAIT_LIMIT_NS)) return;
     *abort = 1;
     *(volatile unsigned*)err = 1;
 }
 // Wait for the barrier's phase, two seconds at most; on a timeout the CTA's
-// abort word is set (every later wait then returns at once and the CTA leaves
-// the kernel at its next tile) and so is the context's error word.
+// abort word is set (every later wait then returns after one look and the CTA
+// leaves the kernel at its next tile) and so is the context's error word.
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort, unsigned* err) {
     if (!mbar_try(bar, parity)) mbar_wait_slow(bar, parity, abort, err);
 }

@@ -1,10 +1,13 @@
 """A wait that makes kernels' results visible to the host also looks at the
 context's error word (sync_checked in csrc/common.cuh), checked without a GPU:
 the helper itself, compiled with g++ against a fake CUDA runtime, and that no
-entry point waits for a stream without it."""
+entry point waits for a stream without it. The kernels' own bounded waits
+(csrc/wait.cuh) run on the host the same way."""
 import os
 import re
 import subprocess
+
+import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "lambda_vm_b200", "csrc")
@@ -33,10 +36,13 @@ def test_waits_go_through_the_checked_helper():
     assert used >= 19
 
 
-def test_the_helper_reports_the_error_word(tmp_path):
-    exe = str(tmp_path / "wait_errors")
+# wait_errors: the helper; bounded_wait: a kernel's wait gives up at its limit,
+# and at once behind another's timeout
+@pytest.mark.parametrize("program", ["wait_errors", "bounded_wait"])
+def test_host_programs(tmp_path, program):
+    exe = str(tmp_path / program)
     r = subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I" + os.path.join(CHOST, "fake_cuda"),
-                        "-I" + os.path.join(ROOT, "include"), os.path.join(CHOST, "wait_errors.cpp"), "-o", exe],
+                        "-I" + os.path.join(ROOT, "include"), os.path.join(CHOST, program + ".cpp"), "-o", exe],
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     run = subprocess.run([exe], capture_output=True, text=True, timeout=60)
