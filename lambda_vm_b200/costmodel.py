@@ -1,7 +1,9 @@
 """Learned cost model of the DFT passes: data, GPU training, tile choice.
 
-The DFT tile width (columns per tile) of every pass is picked at run time
-(csrc/ntt.cu). Without a model the context times each compiled width once on
+The DFT tile width (columns per tile) of a pass on the integer pipes is picked
+at run time (csrc/ntt.cu); passes on the tensor cores (csrc/ntt_tc.cu: most of
+2^7 to 2^11 points above 2^20 in all) have none, are logged with width 0 and
+are no part of the data. Without a model the context times each compiled width once on
 a proxy shape per pass length and scales by the padded column count; that
 probe ranks widths unlike the real passes for some shapes. The model here
 predicts log(ms) of a pass from its shape and width (features: the C
@@ -43,6 +45,11 @@ def tile_widths(log_len):
     if log_len == 11:
         return (4, 8)
     return ()
+
+
+def width_records(records):
+    """The records of passes that had a tile width (not those on the tensor cores)."""
+    return [r for r in records if r["cols"]]
 
 
 def default_width(log_len):
@@ -90,7 +97,9 @@ def sweep_configs(max_cells=1 << 28):
 def collect(be, configs=None, repeats=3, seed=5):
     """Time every config's LDE with each compiled tile width pinned, through
     the pass log; returns {"records": [...], "probe": {log_len: {cols: cost}}}.
-    Each record is one pass (its shape, width and the median ms of `repeats`)."""
+    Each record is one pass (its shape, width and the median ms of `repeats`).
+    A width pins the lengths that have it; what the others of an LDE run on the
+    tensor cores is left out."""
     L = native.lib()
     configs = configs or sweep_configs()
     cols, cost, cnt = (C.c_uint32 * 4)(), (C.c_float * 4)(), C.c_uint32()
@@ -133,6 +142,8 @@ def collect(be, configs=None, repeats=3, seed=5):
                 native.check(L.sg_ctx_pass_log_read(be.h, buf, 64, C.byref(count)))
                 for i in range(count.value):
                     r = buf[i]
+                    if r.cols == 0:
+                        continue
                     rec = {k: int(getattr(r, k)) for k in SHAPE_KEYS}
                     key = (shape_of(rec), int(r.cols), (log_n, m, blowup))
                     recs.setdefault(key, (rec, []))[1].append(float(r.ms))
@@ -165,7 +176,7 @@ def load_dataset(path=DATASET):
         r = dict(zip(d["fields"], row))
         r["lde"] = [r.pop("lde_log_n"), r.pop("lde_m"), r.pop("lde_blowup")]
         recs.append(r)
-    return {"records": recs, "probe": d["probe"]}
+    return {"records": width_records(recs), "probe": d["probe"]}
 
 
 # ---------------------------------------------------------------- split, features
@@ -180,6 +191,7 @@ def split(records, holdout=0.25):
 
 
 def design(records):
+    records = width_records(records)
     X = np.stack([features(r, r["cols"]) for r in records]).astype(np.float32)
     y = np.array([math.log(max(r["ms"], 1e-4)) for r in records], np.float32)
     return X, y
@@ -283,7 +295,7 @@ def evaluate(records, params, probe):
     shapes (ms) and the mean relative regret of the model, the probe rule and
     the fixed default width."""
     by = {}
-    for r in records:
+    for r in width_records(records):
         by.setdefault(shape_of(r), {})[int(r["cols"])] = float(r["ms"])
     tot = {"best": 0.0, "model": 0.0, "probe": 0.0, "default": 0.0}
     reg = {"model": [], "probe": [], "default": []}

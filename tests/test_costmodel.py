@@ -47,6 +47,20 @@ def test_probe_rule_restates_the_tile_chooser():
     assert CM.probe_pick(probe, 9, 40) == 16     # no probe data: the default
 
 
+def test_tensor_core_passes_are_no_width_data(tmp_path):
+    """A pass on the tensor cores is logged with width 0: it is neither trained
+    on nor the width any rule is measured against."""
+    shape = dict(zip(CM.SHAPE_KEYS, (10, 1024, 24, 2, 0, 1, 1, 0)), lde=[20, 24, 2])
+    recs = [dict(shape, cols=c, ms=ms) for c, ms in ((8, 1.2), (16, 1.0), (0, 0.4))]
+    X, y = CM.design(recs)
+    assert X.shape[0] == 2 and list(np.exp(y)) == pytest.approx([1.2, 1.0])
+    ev = CM.evaluate(recs, CM.init_params(1), {"10": {"4": 1.2, "8": 1.1, "16": 1.0}})
+    assert ev["shapes"] == 1 and ev["ms"]["best"] == 1.0 and ev["mean_regret"]["default"] == 0
+    path = str(tmp_path / "d.json")
+    CM.save_dataset({"records": recs, "probe": {}}, path)
+    assert [r["cols"] for r in CM.load_dataset(path)["records"]] == [8, 16]
+
+
 @pytest.mark.skipif(not os.path.exists(CM.MODEL), reason="no committed model")
 def test_committed_model_beats_the_probe_on_heldout_shapes():
     params, meta = CM.load_model()

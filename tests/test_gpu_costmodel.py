@@ -84,3 +84,18 @@ def test_context_with_the_model_chooses_widths_without_probing():
         assert (got == O.canon_array(O.coset_lde_row_major(t, 2, w))).all()
     finally:
         fresh.close()
+
+
+@pytest.mark.parametrize("config", [(15, 128, 2), (21, 9, 2)])
+def test_collected_records_have_a_width(config):
+    """LDEs with passes on the tensor cores whatever is pinned: lengths without
+    a choice (2^7) and, at width 16, 2^11."""
+    from lambda_vm_b200.device import Backend
+    fresh = Backend(0)
+    try:
+        data = CM.collect(fresh, [config], repeats=1)
+    finally:
+        fresh.close()
+    widths = {(r["log_len"], r["cols"]) for r in data["records"]}
+    assert widths == ({(8, 4), (8, 8), (8, 16)} if config[0] == 15 else
+                      {(10, 4), (10, 8), (10, 16), (11, 4), (11, 8)})
