@@ -716,11 +716,11 @@ int sg_eval_constraints(sg_ctx* c, void* stream, const sg_device_program* prog, 
         // one segment; row-major, each read moves a 32-byte sector for 8
         // bytes). The copy moves 2m words a row, so it pays once a row reads
         // at least m operands; skipped when the budget has no room for it.
-        // The KECCAK kernel takes it too; the CPU and SHIFT tables' kernels
-        // read their rows' columns nearly in order, so the rest of each
-        // sector is still in L1 when it is needed, and measured faster
-        // without the copy (with the copy's time: CPU 2^22 rows 24.2 ->
-        // 20.5 ms, SHIFT 2^20 rows 3.53 -> 2.82 ms).
+        // The KECCAK kernel takes it too. The SHIFT table's reads its rows'
+        // columns nearly in order, so the rest of each sector is still in L1
+        // when it is needed: faster without the copy (with the copy's time,
+        // 2^20 rows 3.53 -> 2.82 ms). The CPU table's brings whole row
+        // segments to shared memory and needs no copy.
         uint64_t* d_cm = nullptr;
         const uint64_t cm_bytes = rows * m * 8;
         const bool hand_copy = hand && hand_id == SG_AIR_KECCAK;
@@ -758,8 +758,8 @@ int sg_eval_constraints(sg_ctx* c, void* stream, const sg_device_program* prog, 
                                              comp ? 0 : 1, comp ? d_extra : d_out);
                 rc = check_launch(ctx, "k_keccak_constraints");
             } else if (hand_id == SG_AIR_SHIFT) {
-                k_shift_constraints<<<grid, 128, 0, st>>>(d_cm, d_main, rows, next_step, d_blob + o_beta,
-                                                          comp ? 0 : 1, comp ? d_extra : d_out);
+                k_shift_constraints<<<grid, 128, 0, st>>>(d_cm, d_main, rows, d_blob + o_beta, comp ? 0 : 1,
+                                                          comp ? d_extra : d_out);
                 rc = check_launch(ctx, "k_shift_constraints");
             } else {
                 KernelInfo ki;

@@ -44,16 +44,14 @@ __host__ __device__ constexpr uint32_t cpu_air_constraints(uint32_t chips) {
     return 117 + 4 + absent + 30 + (bw ? 6 : 0) + (mem ? 12 : 0) + 64 + 65;
 }
 
+// A SHIFT-table row, from the column-major copy (cm) or the LDE (rm).
 struct CRow {
     const uint64_t* cm;
     const uint64_t* rm;
-    uint64_t rows, width, row, rn;
-    __device__ __forceinline__ uint64_t at(uint64_t r, uint32_t col) const {
-        return cm ? cm[(uint64_t)col * rows + r] : rm[r * width + col];
+    uint64_t rows, width, row;
+    __device__ __forceinline__ uint64_t M(uint32_t col) const {
+        return cm ? cm[(uint64_t)col * rows + row] : rm[row * width + col];
     }
-    __device__ __forceinline__ uint64_t M(uint32_t col) const { return at(row, col); }
-    __device__ __forceinline__ uint64_t N(uint32_t col) const { return at(rn, col); }
-    __device__ __forceinline__ uint64_t sel(uint32_t op) const { return M(CPU_SEL0 + op - 1); }
 };
 
 __device__ __forceinline__ uint32_t cpu_xlo(uint32_t k) { return CPU_X0 + 2 * (k - 1); }
@@ -282,11 +280,11 @@ constexpr uint32_t SH_DIR = 0, SH_AB = 1, SH_S = 65, SH_Q = 73, SH_TB = 81, SH_R
                    SH_WIDTH = 148, SH_CONSTRAINTS = 149;
 
 static __global__ void k_shift_constraints(const uint64_t* __restrict__ cm, const uint64_t* __restrict__ rm,
-                                           uint64_t rows, uint64_t next_step, const uint64_t* __restrict__ beta,
-                                           int mode, uint64_t* __restrict__ out) {
+                                           uint64_t rows, const uint64_t* __restrict__ beta, int mode,
+                                           uint64_t* __restrict__ out) {
     for (uint64_t row = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; row < rows;
          row += (uint64_t)gridDim.x * blockDim.x) {
-        const CRow w{cm, rm, rows, SH_WIDTH, row, row};
+        const CRow w{cm, rm, rows, SH_WIDTH, row};
         KSink s{beta, mode, out, rows, row, gl::wzero3(), 0};
         const uint64_t d = w.M(SH_DIR), nd = gl::sub(1, d);
         s.put(kbool(d));
