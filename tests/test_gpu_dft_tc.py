@@ -1,6 +1,6 @@
 """DFT passes on the tensor cores (csrc/ntt_tc.cu): LDEs and transforms at the
 edges of its tiles, bit for bit against the CPU oracle. Every case checks, by
-the context's pass log, that passes really ran there."""
+the context's pass log, which passes ran there."""
 import ctypes as C
 
 import numpy as np
@@ -30,6 +30,26 @@ def tensor_passes(be, call):
     return out, [(r.log_len, r.inverse, r.post) for r in rec[:cnt.value] if r.cols == 0]
 
 
+def passes(log_n, m, blowup):
+    """An LDE's passes as (length, inverse, factor) with their points (rows x
+    columns x cosets), in order; blowup 0: a forward transform's, -1: an
+    inverse one's."""
+    n = (1 << log_n) * m
+    halves = [log_n // 2, log_n - log_n // 2] if log_n > 12 else [log_n]
+    if blowup <= 0:
+        inv, last = -blowup, 0 if blowup == 0 else 3
+        kinds = [(halves[0], inv, 1), (halves[-1], inv, last)]
+        return [(k, n) for k in kinds[2 - len(halves):]]
+    kinds = [(halves[0], 1, 1), (halves[-1], 1, 2), (halves[0], 0, 1), (halves[-1], 0, 0)]
+    kept = kinds if len(halves) == 2 else kinds[1::2]
+    return [(k, n * (1 if k[1] else blowup)) for k in kept]
+
+
+def long_passes(log_n, m, blowup):
+    """Those of 2^7 to 2^11 points over more than 2^20 in all."""
+    return [k for k, points in passes(log_n, m, blowup) if 7 <= k[0] <= 11 and points > 1 << 20]
+
+
 # (rows, columns, blowup): pass lengths 2^7..2^11 (2^11 splits into two 2^10
 # transforms), column counts one below, at and one above a tile's 128 / 64 /
 # 32 / 16 / 8 columns, narrow matrices (flat tiles), one to sixteen cosets, single-pass
@@ -44,6 +64,8 @@ def test_lde_matches_oracle(be, log_n, m, blowup):
     t, w = raw(log_n * 1000 + m, (n, m)), O.coset_weights(n, 3)
     got, tc = tensor_passes(be, lambda: mc.coset_lde_batch_base(t, blowup, w, be))
     assert tc, "no pass ran on the tensor cores"
+    # 70 tiles of 2^14 x 70 are too few in a round (below)
+    assert tc == [k for k in long_passes(log_n, m, blowup) if (log_n, m) != (14, 70) or not k[1]]
     assert (got == O.canon_array(O.coset_lde_row_major(t, blowup, w))).all()
 
 
@@ -51,10 +73,11 @@ def test_lde_matches_oracle(be, log_n, m, blowup):
 def test_transforms_match_oracle(be, log_n, m):
     x = raw(log_n * 77 + m, (1 << log_n, m))
     fw, tc = tensor_passes(be, lambda: mc.ntt_forward(x, be))
-    assert {p[1] for p in tc} == {0}
+    assert {p[1] for p in tc} == {0} and tc == long_passes(log_n, m, 0)
     assert (fw == O.canon_array(O.fft(x))).all()
     back, tc = tensor_passes(be, lambda: mc.ntt_inverse(fw, be))
     assert (1, 1) in {p[1:] for p in tc} and (1, 3) in {p[1:] for p in tc}
+    assert tc == long_passes(log_n, m, -1)
     assert (back == O.canon_array(x)).all()
 
 

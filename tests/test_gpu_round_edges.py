@@ -209,3 +209,23 @@ def test_keccak_table_beyond_one_wave(be):
     want = mc.eval_constraints_on_device(dev, main, aux, *rest)
     got = mc.eval_constraints_on_device(dev, np.tile(main, (reps, 1)), np.tile(aux, (reps, 1)), *rest)
     assert np.array_equal(got, np.tile(want, (reps, 1)))
+
+
+# A chunk is at most the 32768 rows whose sums of 255 x 255 an s32 accumulator
+# holds. So many rows that two CTAs an SM would get 66201 each, past 2^32; all
+# bytes of the columns are 255, those of the weights 255 or 254.
+@pytest.mark.parametrize("k", [1, 2])
+def test_barycentric_chunks_of_the_largest_length(be, k):
+    import torch
+    from lambda_vm_b200 import native
+    n, cols = 296 * 66200 + 77, 12
+    data = torch.full((n * cols,), -1, dtype=torch.int64, device="cuda")
+    pts = torch.ones(n, dtype=torch.int64, device="cuda")
+    invd = torch.full((3 * k * n,), P - 2 - (1 << 64), dtype=torch.int64, device="cuda")
+    out = torch.zeros(3 * k * cols, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    native.check(native.lib().sg_barycentric_sums(be.h, None, data.data_ptr(), cols, 1, 0, cols, pts.data_ptr(),
+                                                  invd.data_ptr(), n, k, out.data_ptr()))
+    be.sync()
+    want = n * (P - 2) * (2**64 - 1) % P
+    assert (out.cpu().numpy().view(np.uint64) == np.uint64(want)).all()
