@@ -395,7 +395,13 @@ static bary_fn bary_kernel(uint32_t K) {
 // two points: 811 us in k_bary, 291 here (2.9 TB/s).
 constexpr uint32_t BT_COLS = 80, BT_ROWS = 128, BT_MT = 5, BT_THREADS = 256;
 constexpr uint32_t BT_MAX_CHUNK = 32768;
-constexpr uint64_t BT_MIN_ROWS = 1ULL << 15, BT_MIN_COLS = 12;
+constexpr uint64_t BT_MIN_ROWS = 1ULL << 15;
+// Columns from which these products are the quicker form. 2^15 rows x 12
+// columns, one and two points: 12 and 15 us against 18 and 23 in k_bary; 2^17 x
+// 12: 19 and 22 against 24 and 31; 2^20 x 12, two points: 96 against 117. One
+// point of long tables is bound by the loads of its short rows (2^20 x 12: 92
+// against 77). Below 12 columns and 2^15 rows both take 10 to 40 us.
+inline uint64_t bary_tc_cols(uint64_t n, uint32_t k) { return k == 1 && n >= (1ULL << 19) ? 16 : 12; }
 template <int K>
 struct BaryTc {
     static constexpr uint32_t Q = 3 * K, N = K == 1 ? 32 : 48;  // N: a multiple of 16
@@ -1013,7 +1019,7 @@ int sg_barycentric_sums(sg_ctx* c, void* stream, const uint64_t* d_data, uint64_
         return check_launch(ctx, "k_bary_combine");
     };
     // Base-field columns at one or two points over many rows: tensor cores
-    if (!ext3 && k <= 2 && n >= BT_MIN_ROWS && cols >= BT_MIN_COLS && cols < (1u << 24) && ctx->fault_dev) {
+    if (!ext3 && k <= 2 && n >= BT_MIN_ROWS && cols >= bary_tc_cols(n, k) && cols < (1u << 24) && ctx->fault_dev) {
         const uint64_t tiles = (cols + BT_COLS - 1) / BT_COLS, CT = (cols + tiles - 1) / tiles;
         // two CTAs an SM in all; a chunk is whole turns and fits the accumulators
         uint64_t len = (n * tiles + 295) / 296;

@@ -66,13 +66,15 @@ def test_many_points_z_cost_no_more_than_their_number(be):
     assert ms(8, 1 << 18) < 20 * ms(1 << 21, 1)
 
 
-# From 2^15 rows and 12 base columns on, one or two points: column tiles of at
+# From 2^15 rows and 12 base columns on (16 of 2^19 rows and one point), one or two points: column tiles of at
 # most 80 in groups of 16, turns of 128 rows, chunks of whole turns. Columns,
 # strides and rows that end inside each; bytes of 255 in every place.
 @pytest.mark.parametrize("n,ru,cols,stride,k", [(1 << 15, 12, 12, 1, 1), ((1 << 15) + 1, 20, 17, 2, 2),
                                                 ((1 << 15) + 127, 81, 80, 1, 2), (40000, 81, 81, 1, 1),
                                                 (100001, 170, 161, 1, 2), (1 << 17, 33, 33, 2, 2),
-                                                ((1 << 15) - 1, 16, 16, 1, 2), (1 << 15, 11, 11, 1, 2)])
+                                                ((1 << 15) - 1, 16, 16, 1, 2), (1 << 15, 11, 11, 1, 2),
+                                                (1 << 19, 15, 15, 1, 1), (1 << 19, 16, 16, 1, 1),
+                                                (1 << 19, 12, 12, 1, 2)])
 @pytest.mark.parametrize("ones", [False, True])
 def test_barycentric_sums_of_base_columns(be, n, ru, cols, stride, k, ones):
     rng = np.random.default_rng(n + cols)
