@@ -199,21 +199,7 @@ int sg_ctx_create(int device, uint64_t budget, sg_ctx** out) {
         uint64_t thr = ctx->budget;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
-    void* word = nullptr;
-    void* dev_word = nullptr;
-    cudaError_t e = cudaHostAlloc(&word, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable);
-    if (e == cudaSuccess) {
-        *(unsigned*)word = 0;
-        ctx->fault_host = (volatile unsigned*)word;
-        e = cudaHostGetDevicePointer(&dev_word, word, 0);
-        ctx->fault_dev = (unsigned*)dev_word;
-    }
-    if (e != cudaSuccess) {
-        if (word) cudaFreeHost(word);
-        delete ctx;
-        set_error(std::string("context error word: ") + cudaGetErrorString(e));
-        return e == cudaErrorMemoryAllocation ? SG_ERR_OOM : SG_ERR_CUDA;
-    }
+    alloc_fault_word(ctx);
     *out = reinterpret_cast<sg_ctx*>(ctx);
     return SG_OK;
 }

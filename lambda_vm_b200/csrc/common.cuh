@@ -115,8 +115,9 @@ struct Ctx {
     // Learned pass-cost model (mlp.cu): when set, DFT tile widths are its choice.
     std::vector<float> pass_model;
     // One page-locked word that a kernel sets when a bounded wait of its ran
-    // out (ntt_tc.cu, rounds.cu k_bary_tc); null in contexts that do not
-    // allocate. Every launch check and every wait that makes results visible
+    // out (ntt_tc.cu, rounds.cu k_bary_tc). Null in contexts that do not allocate
+    // and where there is no page-locked memory; those run the kernels without
+    // such waits. Every launch check and every wait that makes results visible
     // to the host reports it, from then on: which results are spoiled is not
     // known, so the word is never cleared.
     volatile unsigned* fault_host = nullptr;
@@ -198,6 +199,23 @@ struct KernelInfo {
     int blocks_per_sm = 0;
 };
 int kernel_info(const void* fn, size_t smem, int threads, KernelInfo* out);
+
+// The context's error word, or none when page-locked memory cannot be had.
+inline void alloc_fault_word(Ctx* ctx) {
+    void *word = nullptr, *dev = nullptr;
+    if (cudaHostAlloc(&word, sizeof(unsigned), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (cudaHostGetDevicePointer(&dev, word, 0) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeHost(word);
+        return;
+    }
+    *(unsigned*)word = 0;
+    ctx->fault_host = (volatile unsigned*)word;
+    ctx->fault_dev = (unsigned*)dev;
+}
 
 // An earlier kernel of the context gave up a bounded wait: its output is not valid.
 inline int check_fault(Ctx* ctx) {

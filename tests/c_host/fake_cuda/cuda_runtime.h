@@ -17,4 +17,8 @@ cudaError_t cudaGetDevice(int* device);
 cudaError_t cudaSetDevice(int device);
 cudaError_t cudaGetLastError(void);
 cudaError_t cudaStreamSynchronize(cudaStream_t stream);
+enum { cudaHostAllocPortable = 1, cudaHostAllocMapped = 2 };
+cudaError_t cudaHostAlloc(void** host, size_t bytes, unsigned flags);
+cudaError_t cudaHostGetDevicePointer(void** dev, void* host, unsigned flags);
+cudaError_t cudaFreeHost(void* host);
 const char* cudaGetErrorString(cudaError_t e);

@@ -21,6 +21,24 @@ cudaError_t cudaStreamSynchronize(cudaStream_t) {
     return g_sync_result;
 }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
+// page-locked memory: the calls that succeed, and the words held
+static int g_host_calls_ok = 0, g_words = 0;
+static unsigned g_word = 77;
+cudaError_t cudaHostAlloc(void** host, size_t, unsigned) {
+    if (g_host_calls_ok-- <= 0) return cudaErrorMemoryAllocation;
+    ++g_words;
+    *host = &g_word;
+    return cudaSuccess;
+}
+cudaError_t cudaHostGetDevicePointer(void** dev, void* host, unsigned) {
+    if (g_host_calls_ok-- <= 0) return cudaErrorMemoryAllocation;
+    *dev = host;
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void*) {
+    --g_words;
+    return cudaSuccess;
+}
 
 namespace sg {
 static thread_local std::string g_err;
@@ -54,6 +72,15 @@ int main() {
     b.fail_wait_after.store(3);
     for (int i = 0; i < 3; ++i) EXPECT(sg::check_launch(&b, "k") == SG_OK);
     EXPECT(sg::sync_checked(&b, nullptr, "x") == SG_ERR_CUDA);
+    // no page-locked memory: a context without the word, and none left behind
+    for (int calls = 0; calls < 3; ++calls) {
+        sg::Ctx c;
+        g_host_calls_ok = calls, g_words = 0;
+        sg::alloc_fault_word(&c);
+        EXPECT((c.fault_host != nullptr) == (calls == 2) && (c.fault_dev != nullptr) == (calls == 2));
+        EXPECT(g_words == (calls == 2 ? 1 : 0) && (calls < 2 || *c.fault_host == 0));
+        EXPECT(sg::check_launch(&c, "k") == SG_OK);
+    }
     // a CUDA error of the wait itself is reported as before
     g_sync_result = cudaErrorInvalidDevice;
     EXPECT(sg::sync_checked(&none, nullptr, "prove") == SG_ERR_CUDA);
