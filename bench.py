@@ -845,14 +845,17 @@ def main():
         traffic_src = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of the 4 k_dft_tc launches of "
                        "one 2^20 x 16 blowup-4 LDE, x m/16 (profiles/k_dft_tc_coset_lde_1048576x16_blowup4.md)")
     achieved = alg[dom] / (med[dom] * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": {"lde": "k_dft_tc (coset LDE, 4 launches)", "leaves": "k_leaves",
-                                          "tree": "k_merkle_levels"}[dom],
+    # frac is of the HBM copy rate; no unit is full in the LDE's passes (their
+    # loads, products and arithmetic overlap too little), Keccak fills the ALU pipe
+    roofline = {"bound": {"lde": "latency", "leaves": "int", "tree": "int"}[dom],
+                "kernel": {"lde": "k_dft_tc (coset LDE, 4 launches)", "leaves": "k_leaves",
+                           "tree": "k_merkle_levels"}[dom],
                 "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
                 "peak_source": peak_src, "traffic": traffic, "traffic_source": traffic_src,
                 "per_kernel_ms": {k: round(v, 3) for k, v in med.items()},
                 "per_kernel_gbs": {k: round(alg[k] / (med[k] * 1e-3) / 1e9, 1) for k in med},
-                "note": "DFT passes are exact u8 products on the tensor cores with INT-pipe recombination, Keccak runs "
-                        "on the INT pipes; see profiles/ for issue utilisation",
+                "note": "DFT passes are exact u8 products on the tensor cores with INT-pipe recombination, no unit full; "
+                        "Keccak fills the ALU pipe; frac is of the HBM copy rate; see profiles/ for utilisation",
                 "int_pipes": {"issue_active_frac": 0.410,
                               "thread_instr_per_point": {"I1": 110, "I2": 117, "F1": 107, "F2": 89},
                               "source": "ncu, the 4 k_dft_tc launches of a 2^20 x 16 blowup-4 LDE, time-weighted "
