@@ -122,16 +122,20 @@ SG_API int sg_ntt_inverse(sg_ctx* ctx, void* stream, uint64_t* d_data, uint64_t 
 SG_API int sg_coset_lde(sg_ctx* ctx, void* stream, const uint64_t* d_trace, uint64_t n, uint64_t m, uint32_t blowup,
                  const uint64_t* d_weights, uint64_t* d_out);
 /* ---- DFT tile autotuning (no reference counterpart: the reference fixes its
- *      kernels' launch shapes). Each pass of 2^log_len points can run with
- *      several compiled tile widths (columns per tile; 4/8/16 for lengths
+ *      kernels' launch shapes). Passes of 2^7..2^11 points over more than 2^20
+ *      points (rows x columns x cosets) run on the tensor cores where that is
+ *      quicker and have no width; this is about the others, on the integer
+ *      pipes, and about lengths pinned below. Each such pass of 2^log_len points
+ *      can run with several compiled tile widths (columns per tile; 4/8/16 for lengths
  *      2^8..2^10, 4/8 for 2^11). On a context's first pass of a length, every
  *      width is timed on the same work and its time per column kept; a pass
  *      over m columns then uses the width minimising ceil(m/C)*C*cost(C),
  *      keeping the default width (16 up to 2^10, 8 at 2^11) unless another is
  *      at least 3 % cheaper; a context with a learned pass-cost model
  *      (sg_ctx_set_pass_model, below) predicts each width's pass time instead
- *      and never times. Results never depend on the width. sg_ctx_dft_tiles pins a width for a
- *      length (cols = 0: automatic); sg_ctx_dft_tuning reports the widths and
+ *      and never times. Results never depend on the width or the kernel.
+ *      sg_ctx_dft_tiles pins a width for a length, whose passes then all stay on
+ *      the integer pipes (cols = 0: automatic); sg_ctx_dft_tuning reports the widths and
  *      their time per column (ms), timing them on `stream` first if needed. ---- */
 SG_API int sg_ctx_dft_tiles(sg_ctx* ctx, uint32_t log_len, uint32_t cols);
 SG_API int sg_ctx_dft_tuning(sg_ctx* ctx, void* stream, uint32_t log_len, uint32_t* cols, float* cost_per_col,
@@ -226,8 +230,8 @@ typedef struct sg_table_desc {
 SG_API int sg_batch_commit(sg_ctx* ctx, void* stream, const sg_table_desc* tables, uint32_t count,
                            uint32_t concurrency, sg_lde** out_ldes, uint8_t* roots_out);
 /* The same commitments with the tables' LDEs fused: every pass of every table
- * goes into one persistent multi-table DFT launch per (step, pass length,
- * tile width, direction), so small tables share the grid with large ones
+ * on the integer pipes goes into one persistent multi-table DFT launch per
+ * (step, pass length, tile width, direction), so small tables share the grid with large ones
  * instead of running as launches of a few CTAs (4 steps x a few launches in
  * all, against 4 per table). Each table's leaves and tree follow, heaviest
  * first over `concurrency` streams that start when the LDEs are done.
@@ -678,7 +682,8 @@ SG_API int sg_ctx_pass_log_read(sg_ctx* ctx, sg_pass_record* out, uint32_t capac
  *      (SG_MLP_IN inputs, two hidden layers of SG_MLP_HIDDEN ReLU units, one
  *      output) predicts log(ms) of a DFT pass from its shape and tile width;
  *      trained on the GPU by these kernels from pass-log measurements, it then
- *      chooses each pass's tile width in place of the timing probe.
+ *      chooses the tile width of each pass on the integer pipes in place of the
+ *      timing probe.
  *      Parameters are fp32, laid out W1[H][IN], b1[H], W2[H][H], b2[H], w3[H], b3.
  *      _loss_grad: mean squared error over n samples (x: n x SG_MLP_IN row-major,
  *      y: n targets) and its gradient, one forward and backward pass, reduced in a
@@ -686,8 +691,8 @@ SG_API int sg_ctx_pass_log_read(sg_ctx* ctx, sg_pass_record* out, uint32_t capac
  *      (lr, beta1 0.9, beta2 0.999, eps 1e-8), params updated in place; the final
  *      loss is written to loss_out. _predict: y = model(x). All device pointers.
  *      sg_ctx_set_pass_model installs host-side parameters in the context (count
- *      = SG_MLP_PARAMS; count 0 removes them): pass tile widths are then the
- *      model's choice, and the timing probe never runs. ---- */
+ *      = SG_MLP_PARAMS; count 0 removes them): tile widths are then the model's
+ *      choice, and the timing probe never runs. ---- */
 #define SG_MLP_IN 16
 #define SG_MLP_HIDDEN 32
 #define SG_MLP_PARAMS (SG_MLP_HIDDEN * SG_MLP_IN + SG_MLP_HIDDEN + SG_MLP_HIDDEN * SG_MLP_HIDDEN + SG_MLP_HIDDEN + \

@@ -319,7 +319,8 @@ def evaluate(records, params, probe):
 
 
 def install(be, params):
-    """Hand the parameters to the context: its DFT tile widths become the model's choice."""
+    """Hand the parameters to the context: its DFT tile widths (of passes that are not on the
+    tensor cores) become the model's choice."""
     p = np.ascontiguousarray(params, np.float32)
     native.check(native.lib().sg_ctx_set_pass_model(be.h, p.ctypes.data_as(C.POINTER(C.c_float)), p.size))
 

@@ -112,7 +112,8 @@ struct Ctx {
     std::atomic<bool> passlog_on{false};
     std::mutex passlog_mu;
     std::vector<PassLog> passlog;
-    // Learned pass-cost model (mlp.cu): when set, DFT tile widths are its choice.
+    // Learned pass-cost model (mlp.cu): when set, the tile widths of DFT passes
+    // on the integer pipes are its choice.
     std::vector<float> pass_model;
     // One page-locked word that a kernel sets when a bounded wait of its ran
     // out (ntt_tc.cu, rounds.cu k_bary_tc). Null in contexts that do not allocate

@@ -63,7 +63,7 @@ __device__ __forceinline__ uint32_t cpu_xlo(uint32_t k) { return CPU_X0 + 2 * (k
 // thread a row, reading its row's columns straight from the LDE, touched 32
 // rows' sectors per load and waited for them. 2^20 rows: 3.0 ms that way, 3.1
 // with a tile loaded through registers (row by row, each waiting for the
-// last), 2.5 here; two tiles an SM, a third of the issue slots used, the rest
+// last), 2.5 here; two tiles an SM, 39 % of the issue slots used, the rest
 // waits on the copies and at the tile's barriers.
 constexpr uint32_t CPU_TILE = 32, CPU_WARPS = 8, CPU_PITCH = CPU_TILE + 1;
 // The columns read of the next frame row: pc, timestamp, the register file.

@@ -387,8 +387,8 @@ static bary_fn bary_kernel(uint32_t K) {
 // (byte b, column c) of 16 columns, N = (q, a), K = rows. Both operands want
 // the rows' bytes side by side, so a thread takes 16 rows of one column,
 // transposes their bytes (64 byte permutes) and stores 16-byte pieces; the
-// products themselves are free. About 7 instructions a cell where k_bary's
-// multiply-accumulates take 54 at K = 2. A CTA takes a column tile of at most
+// products themselves are free. 30 instructions a cell in all (7 of them the
+// transposition) where k_bary's multiply-accumulates alone take 54 at K = 2. A CTA takes a column tile of at most
 // 80 columns (five M-tiles, 240 TMEM columns) and a chunk of rows; two CTAs
 // share an SM, one loading while the other's products run. The accumulators
 // hold 2^31 / 255^2 > 32768 rows. 2^19 points x 200 columns (every second row),

@@ -52,8 +52,9 @@ class Backend:
 
 def backend(device: int = 0) -> Backend:
     """Process-wide context for `device` (device::backend()). The committed
-    DFT pass-cost model (costmodel.py) chooses its tile widths, unless the
-    environment sets SG_PASS_MODEL=0 (the timing probe then decides)."""
+    DFT pass-cost model (costmodel.py) chooses the tile widths of its passes on
+    the integer pipes, unless the environment sets SG_PASS_MODEL=0 (the timing
+    probe then decides)."""
     import os
     with _lock:
         b = _backends.get(device)
