@@ -104,15 +104,23 @@ __device__ fe3 deep_at(const sg_verify_table& T, uint64_t x, const uint64_t* rm,
     const uint64_t* C = T.consts;
     const uint32_t m = T.m, W = T.m + T.aux_cols;
     const fe3 z = c3(C, 0), zw = c3(C, 1), z2 = c3(C, 2);
-    fe3 ah{0, 0, 0}, a0{0, 0, 0}, a1{0, 0, 0};
+    fe3 ah{0, 0, 0};
     for (int j = 0; j < 2; ++j)
         ah = gl::add3(ah, gl::mul3(c3(C, 3 + j), gl::sub3(c3(rp, j), c3(C, 5 + j))));
+    // The columns' sums stay unreduced: a thread has a query to itself, so the
+    // length of its chain of products is its time (6 accumulators in flight
+    // here where two Fp3 products and their reductions were in line).
+    gl::wacc3 s0 = gl::wzero3(), s1 = gl::wzero3();
+    auto mac = [](gl::wacc3& s, const fe3& g, const fe3& v) {
+        gl::wmac3(s, g, v, gl::add(v.c1, v.c1), gl::add(v.c2, v.c2));
+    };
     const uint64_t gt0 = 7, td0 = 7 + 2ull * W;
     for (uint32_t j = 0; j < W; ++j) {
         const fe3 tv = j < m ? base3(rm[j]) : c3(ra, j - m);
-        a0 = gl::add3(a0, gl::mul3(c3(C, gt0 + 2ull * j), gl::sub3(tv, c3(C, td0 + j))));
-        a1 = gl::add3(a1, gl::mul3(c3(C, gt0 + 2ull * j + 1), gl::sub3(tv, c3(C, td0 + W + j))));
+        mac(s0, c3(C, gt0 + 2ull * j), gl::sub3(tv, c3(C, td0 + j)));
+        mac(s1, c3(C, gt0 + 2ull * j + 1), gl::sub3(tv, c3(C, td0 + W + j)));
     }
+    const fe3 a0 = gl::wreduce3(s0), a1 = gl::wreduce3(s1);
     const fe3 ih = gl::inv3(gl::sub3(base3(x), z2));
     const fe3 i0 = gl::inv3(gl::sub3(base3(x), z));
     const fe3 i1 = gl::inv3(gl::sub3(base3(x), zw));
